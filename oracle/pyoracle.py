@@ -25,6 +25,8 @@ LIB_REF = os.path.join(HERE, "_ref", "libpbref.so")
 # this repository
 REFERENCE_DIR = os.environ.get(
     "PB_REFERENCE_DIR", os.path.normpath(os.path.join(HERE, os.pardir, os.pardir, "reference")))
+if not os.path.exists(os.path.join(REFERENCE_DIR, "kernelfuncs.cu")):
+    REFERENCE_DIR = ""  # no checkout, or a directory without the sources
 
 _u32p = np.ctypeslib.ndpointer(np.uint32, flags="C_CONTIGUOUS")
 _f32p = np.ctypeslib.ndpointer(np.float32, flags="C_CONTIGUOUS")
