@@ -108,6 +108,13 @@ __device__ __forceinline__ void load_v(const IntegrateArgs &a, const SysInt &S, 
   }
 }
 
+// acc + m |v|^2 with every rounding written out: the steps and k_mv2 add the
+// same terms, so a temperature read after a step gives the same bits whichever
+// kernel summed it (left to the compiler, their contractions differed).
+__device__ __forceinline__ double add_mv2(double acc, float m, double x, double y, double z) {
+  return __fma_rn((double)m, __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))), acc);
+}
+
 __global__ void __launch_bounds__(kIntThreads) k_vv(IntegrateArgs a) {
   pdl_enter();
   __shared__ double red[32];
@@ -134,7 +141,7 @@ __global__ void __launch_bounds__(kIntThreads) k_vv(IntegrateArgs a) {
     if (a.wrap) wrap3(S, p);
     a.v[i] = v;
     a.r[i] = p;
-    mv2 += (double)a.mass[i] * ((double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z);
+    mv2 = add_mv2(mv2, a.mass[i], v.x, v.y, v.z);
   }
   double s[1] = {mv2}, tot[1];
   block_sum<1>(s, red);
@@ -270,12 +277,11 @@ __global__ void __launch_bounds__(kIntThreads) k_gauss_b(IntegrateArgs a) {
         a.r[i] = q;
         if (a.vd) {
           store_vd(a, S, i, v);
-          mv2 += (double)g[j].mass * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+          mv2 = add_mv2(mv2, g[j].mass, v[0], v[1], v[2]);
         } else {
           const float4 vf = make_float4((float)v[0], (float)v[1], (float)v[2], 0.f);
           a.v[i] = vf;
-          mv2 += (double)g[j].mass *
-                 ((double)vf.x * vf.x + (double)vf.y * vf.y + (double)vf.z * vf.z);
+          mv2 = add_mv2(mv2, g[j].mass, vf.x, vf.y, vf.z);
         }
       }
     }
@@ -309,7 +315,7 @@ __global__ void __launch_bounds__(kIntThreads) k_mv2(IntegrateArgs a) {
     const uint32_t i = m.i0 + t;
     double v[3];
     load_v(a, S, i, v);
-    s[0] += (double)a.mass[i] * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+    s[0] = add_mv2(s[0], a.mass[i], v[0], v[1], v[2]);
   }
   double tot[1];
   block_sum<1>(s, red);

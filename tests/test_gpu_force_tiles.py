@@ -1,0 +1,102 @@
+"""The tiled force kernel at the edges of its tiles, blocks and tables, against
+all pairs in FP64: partial and single-atom tiles, empty cells, columns of one
+and of many runs, cells wider than the cutoff (more candidate blocks than the
+warps' table holds), one to five atom types with their own cutoffs, 64-bit
+sums, open boxes, and atoms far outside their cells."""
+import numpy as np
+import pytest
+
+from particlebase_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+BAR = 1e-5  # relative RMS of the forces, the bar of the plain FP32 path
+
+
+def system(L, n, ntypes, seed):
+    """n atoms on a jittered grid of spacing 1.12 or more in a box of edges L."""
+    rng = np.random.default_rng(seed)
+    L = np.asarray(L, np.float32).astype(np.float64)
+    k = np.floor(L / 1.12).astype(int)
+    g = np.stack(np.meshgrid(*[np.arange(x) for x in k], indexing="ij"), -1).reshape(-1, 3)
+    g = g[rng.permutation(len(g))[:n]]
+    r = (g + 0.5 + rng.uniform(-0.12, 0.12, g.shape)) * (L / k)
+    r = r.astype(np.float32).astype(np.float64)
+    lj = np.zeros((ntypes, ntypes, 3))
+    for a in range(ntypes):
+        for b in range(ntypes):
+            sig = 0.5 * (1.0 - 0.04 * a + 1.0 - 0.04 * b)
+            lj[a, b] = sig, 1.0 + 0.1 * abs(a - b), 2.5 * sig
+    lj = lj.astype(np.float32).astype(np.float64)
+    box = np.array([0, L[0], 0, L[1], 0, L[2]], np.float32)
+    types = rng.integers(0, ntypes, len(r)).astype(np.uint32)
+    return W.LJSystem(box=box, r=r, v=np.zeros_like(r), mass=np.ones(len(r)), types=types, lj=lj,
+                      rc=2.5)
+
+
+def all_pairs(s, periodic=True):
+    d = s.r[:, None] - s.r[None]
+    if periodic:
+        d -= s.L * np.round(d / s.L)
+    r2 = (d ** 2).sum(-1)
+    sig, eps, rc = np.moveaxis(s.lj[s.types[:, None], s.types[None]], -1, 0)
+    near = (r2 < rc * rc) & (r2 > 0)
+    r2 = np.where(near, r2, 1.0)
+    s6 = (sig * sig / r2) ** 3
+    f = np.where(near, 24 * eps * s6 * (2 * s6 - 1) / r2, 0.0)
+    pe = np.where(near, 4 * eps * s6 * (s6 - 1), 0.0).sum() / 2
+    return (f[..., None] * d).sum(1), pe
+
+
+def check(s, periodic=True, rmax=2.5, **kw):
+    from particlebase_b200.md import from_system
+    p = from_system(s, cell_rmax=rmax, **kw)
+    if not periodic:
+        p.setupCutoffBlock(rmax, periodic=False)
+    p.calcBlockID()
+    F, pe = all_pairs(s, periodic)
+    scale = max(np.sqrt((F ** 2).sum()), 1.0)
+    for energy in (False, True):
+        p.calcForce(energy=energy)
+        got = p.get("F")[:, :3].astype(np.float64)
+        assert np.sqrt(((got - F) ** 2).sum()) < BAR * scale
+    assert abs(p.sums()["pe"] - pe) < BAR * max(abs(pe), 1.0)
+    return p.status()
+
+
+@pytest.mark.parametrize("L,n", [
+    ((7.9, 7.9, 7.9), 1), ((7.9, 7.9, 7.9), 2), ((7.9, 8.2, 9.0), 15), ((7.9, 8.2, 9.0), 16),
+    ((7.9, 8.2, 9.0), 17), ((7.9, 8.2, 9.0), 343), ((8.0, 13.0, 40.0), 33),
+    ((8.0, 8.0, 60.0), 1500), ((20.0, 8.0, 8.0), 800), ((11.0, 10.4, 18.1), 1201)])
+def test_one_type(cuda_lib, L, n):
+    assert check(system(L, n, 1, n)) == 0
+
+
+@pytest.mark.parametrize("ntypes", [2, 3, 4, 5, 8])
+def test_types_with_their_own_cutoffs(cuda_lib, ntypes):
+    assert check(system((9.0, 10.5, 16.0), 900, ntypes, ntypes)) == 0
+
+
+@pytest.mark.parametrize("ntypes", [1, 2])
+def test_64_bit_sums(cuda_lib, ntypes):
+    assert check(system((9.0, 10.5, 16.0), 701, ntypes, 7), fp64_forces=True) == 0
+
+
+@pytest.mark.parametrize("rmax,ntypes", [(4.9, 1), (4.9, 3), (3.7, 2)])
+def test_cells_wider_than_the_cutoff(cuda_lib, rmax, ntypes):
+    assert check(system((15.0, 15.0, 15.0), 2100, ntypes, 3), rmax=rmax) == 0
+
+
+@pytest.mark.parametrize("far", [0.0, 30.0, 4000.0])
+def test_open_box_and_atoms_far_outside(cuda_lib, far):
+    """Past some hundred cell edges an atom leaves the range of the stage's fp16
+    records, and the items that stage it compute from global memory."""
+    s = system((12.0, 11.0, 14.0), 700, 1, 5)
+    if far:
+        s.r[3] = (-far, 4.0, 5.0)
+        s.r[90] = (3.0, -0.4, 2.0)
+        s.r = s.r.astype(np.float32).astype(np.float64)
+        d = s.r - s.r[90]
+        keep = ((d ** 2).sum(1) > 0.9) | (np.arange(s.n) == 90)  # no overlap with the moved atom
+        s.r, s.v, s.mass, s.types = s.r[keep], s.v[keep], s.mass[keep], s.types[keep]
+    assert check(s, periodic=False) == 0
