@@ -9,27 +9,19 @@
 // (r_i - r_j) with the minimum image, over the 27-cell stencil.  No 81 N
 // scratch: each atom's force is summed in registers and written once.
 //
-// Work items.  One work item = (system, x-y column of cells, run of z cells
-// [z0, z1)); its stage is the 3 x 3 neighbour columns over z cells
-// [z0 - 1, z1] (periodic halo cells included).
-//
-// Persistent, warp-specialised CTAs.  Each CTA walks the items blockIdx.x,
-// blockIdx.x + gridDim.x, ... with two stage buffers.  Warp 0 is the
-// producer: for item n + 1 it reads the cell starts, lands the stage in the
-// free buffer with 1-D bulk copies (cp.async.bulk, mbarrier completion, no
-// multicast) from the structure-of-arrays mirrors of the sorted positions,
-// applies the frame shifts, and searches the z window of every (cluster,
-// column).  The other warps are consumers: they compute item n from the other
-// buffer meanwhile, and move on to item n + 1 as soon as the producer
-// publishes it.  mbarriers hand buffers back and forth (full: producer to
-// consumers; empty: consumers to producer); every wait is bounded.
-//
-// Stage layout.  Each staged column is a run of whole 4-atom quads: the bulk
-// copies move 16-byte aligned runs of the x, y, z (and type) mirrors, so up to
-// 3 atoms of the neighbouring cells ride along at each end of a run; the
-// producer turns those into far atoms (x, y = 1e30) whose z keeps the column
-// sorted.  Mirror runs start at the same offset modulo 4 whether a system runs
-// alone or in a batch, so the layout, and every sum, is the same in both.
+// Work items.  One CTA of 8 warps computes one work item = (system, x-y column
+// of cells, run of z cells [z0, z1)), about 8 tiles of 16 consecutive
+// (z-sorted) home atoms.  It stages the 3 x 3 neighbour columns over z cells
+// [z0 - 1, z1] (periodic halo cells included) in shared memory by bulk copies
+// of the sorted positions (bounded wait), then a warp takes a tile and waits
+// for no other.  Four CTAs share an SM, so one's staging overlaps another's
+// computation.  What bounds it is instruction issue (70 % of the slots at 1M
+// atoms, shared memory 58 %).  Per home atom 182 warp instructions: staging 30,
+// block tables 23, phase 1 56, phase 2 73.  Longer runs stage fewer halo cells
+// per home atom and shorter ones fit more CTAs: 4, 5, 6 and 7 cells of 14 atoms
+// took 0.362, 0.322, 0.284 and 0.268 ms at 1M atoms; 9 cells, at three CTAs per
+// SM, 0.293; CTAs of 16 warps over 14 cells 0.281.  A persistent kernel with
+// producer warps that tested quads of candidates with FMAs took 0.325 ms.
 //
 // Coordinate frame.  Positions are absolute FP32 coordinates.  Each item moves
 // all staged atoms into one frame by subtracting 0 or L per axis: a neighbour
@@ -38,27 +30,44 @@
 // coordinates >= L/2, where it is exact (Sterbenz), so displacements x_i - x_j
 // in the frame are the minimum-image displacements with no rounding beyond
 // the subtraction itself, even in a 190-sigma box.  Work items are laid out
-// so that a top-face item's cells all lie above the box middle.
+// so that a top-face item's cells all lie above the box middle (a column that
+// fits one run rounds only the image above its top).
 //
-// Compute.  Cells are sorted by z and atoms within a cell by z, so every
-// staged column is one z-sorted array.  A consumer warp takes a cluster of 8
-// consecutive home atoms (lane & 7) and splits the candidates 4 ways
-// (lane >> 3).  It writes the quads of the cluster's 9 column windows into one
-// flat table (padded to whole chunks with a quad of far atoms), so the
-// candidate loop runs over one sequence with no per-column tails.  Then
-//   phase 1  tests 4 candidates per step (one quad, packed FP32x2 arithmetic)
-//            against rc^2 (1 + 2^-10) and appends the hits to a per-lane index
-//            list in shared memory (no divergent force code);
-//   phase 2  recomputes each listed pair exactly, applies the exact cutoff
-//            r^2 < rc^2 of the pair's types (which also drops the self pair,
-//            r^2 = 0), and evaluates the force, two list entries per step in
-//            packed FP32x2 arithmetic.
-// The 4 partial sums of an atom are combined with two warp shuffles.
-// Clusters go to consumers round-robin over the CTA's whole item sequence;
-// a cluster's arithmetic does not depend on which warp runs it, and energy
-// sums are kept per cluster and added in cluster order.  An item whose stage
-// exceeds the shared-memory capacity computes from global memory instead
-// (slower, same result) and raises a status bit.
+// Stage.  Each staged column is one z-sorted array padded with far atoms
+// (coordinates 1e30) to a multiple of 8 slots.  A slot holds the exact frame
+// position and type (16 B), and an approximate record of four fp16 values (8 B):
+// the position relative to the item's centre in units of the longest cell edge,
+// and its squared norm; with several types also the indicators of its type.
+//
+// Phase 1, on the tensor cores.  The candidates of a tile are the blocks of 8
+// whose z range meets [zmin - rc, zmax + rc].  One mma.sync m16n8k8 (fp16
+// operands, FP32 sums) gives 16 x 8 values
+// |x_j|^2 - 2 x_i . x_j + (|x_i|^2 - bound), whose sign says whether the pair
+// may be within rc.  `bound` exceeds rc^2 by what the rounding of the records
+// can change (from the largest norm staged), so the hits are a superset of the
+// pairs inside the cutoff: about 4 % more.  With several types the indicators'
+// share of the product lowers the bound to that pair of types' own cutoff.
+// mma.sync and not tcgen05: a tile shares its window with no other, its product
+// has a depth of 8, and 52 of them take 8 % of the tensor pipe; the work is in
+// reading their signs.  A lane owns 2 home atoms x 2 candidates of each block
+// and lists the candidates that may be near either of its two.
+//
+// Phase 2.  Each lane walks its list (lane-minor in shared memory).  It fetches
+// the exact position once, evaluates the pairs with both its home atoms
+// (neighbours in z, sharing most candidates: 1.42 sphere volumes for 2) in
+// packed FP32x2 arithmetic, each home atom one half, and applies the exact
+// cutoff 0 < r^2 < rc^2 (the self pair has r^2 = 0).  Two shuffles combine the 4
+// lanes of an atom.  Bit strings in registers instead of lists cost 51
+// instructions a step against 38 (0.364 against 0.325 ms with the staging of
+// that version); evening out the lists of neighbouring lanes gained nothing.
+//
+// Every sum runs in candidate order within a lane and in a fixed order over
+// the lanes, and windows and blocks depend on the item alone, so a system's
+// forces do not depend on scheduling or on the other systems of a batch.  An
+// item whose stage exceeds its capacity computes from global memory instead
+// (slower) and raises a status bit.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <type_traits>
 
@@ -67,58 +76,54 @@
 namespace pb {
 namespace {
 
-// One work item as the consumers see it (written by the producer).
+constexpr int kTile = 16;         // home atoms per tile (rows of one mma)
+constexpr int kTabBlocks = 96;    // blocks in a warp's table at once
+constexpr uint32_t kTabBytes = kTabBlocks * 4;
+// Hits a lane lists before they are evaluated: as many as leave the shared
+// memory for the CTAs per SM that the registers allow.
+__host__ __device__ constexpr uint32_t list_len(int nt) { return nt > 1 ? 36u : 28u; }
+// Per warp: the table of block starts, and the lanes' lists of hits.
+__host__ __device__ constexpr uint32_t warp_bytes(int nt) { return kTabBytes + list_len(nt) * 64u; }
+constexpr float kMaxNorm = 30000.f;  // largest norm the fp16 records are used for
+
+// One work item: its staged columns and the constants of its frame.
 template <int NT>
-struct ItemDesc {
-  // index within column c of the first staged atom of z cell k (k = 0 is image
-  // cell z0 - 1, k = nseg + 1 is image cell z1); entry nseg + 2 is the column's count
-  uint32_t off[9][kMaxSeg + 3];
-  uint32_t ps[10];     // first slot of each column's region; ps[9] = end
-  uint32_t kbase[9];   // packed key of z cell 0 of each column
-  float sx[9], sy[9];  // frame shift of each column (0 or L)
-  float sz_lo, sz_mid, sz_hi;  // frame shift of staged cell 0, 1..nseg, nseg + 1
-  uint32_t item, sys, home_g0, hb, H, nclus, ntask, sentinel, base;
-  int z0, nz, nseg;
-  int periodic;        // 0: open box (neighbour columns may be absent, no z images)
-  int skip;            // the system's step budget is spent
-  int overflow;        // the stage exceeds the capacity: global-memory path
+struct Stage {
+  uint32_t c0[10];        // first slot of each column's region (multiples of 8); c0[9] = end
+  uint32_t e0[9], e1[9], e2[9];  // ends of its low image, middle run and high image
+  float sx[9], sy[9];     // frame shift of each column (0 or L)
+  float szl, szm, szh;    // frame shift of the low image, the middle run, the high image
+  float cx, cy, cz, scale;  // centre and scale of the fp16 records
+  float rcw;              // half-width of the z windows
+  float rs2;              // rc^2 (of the longest-ranged pair) in record units
+  uint32_t home_g0, hb, H, ntile;  // home atoms: first sorted slot, first stage slot, count
+  uint32_t kbase[9];
+  int z0, nz, nseg, periodic, overflow;
+  int shifted;            // some frame shift is not zero
+  uint32_t nmax;          // largest norm staged (float bits, non-negative)
   LJLocal<NT> lj;
-  // z window of each (cluster, column): first quad, quads, flat offset; per
-  // cluster the total and the longest (at least 2)
-  uint16_t q0[kWinCap][9], len[kWinCap][9], pre[kWinCap][9];
-  uint16_t Q[kWinCap], M[kWinCap];
+  // several types: what the bound of a pair of types lies below the longest
+  // one, per type of home atom as fp16 for candidate types 0 .. 3
+  uint2 cut[NT > 1 ? NT : 1];
+  float4 lj4[NT > 1 ? NT * NT : 1];  // {sigma^2, 24 eps, bits of rc^2 less one, 0} per type pair
 };
 
-// Producer scratch: global cell starts and counts of the item being staged,
-// and its copy runs (piece p of column c at index 3 c + p).
-struct Scratch {
-  uint32_t gstart[9][kMaxSeg + 3];
-  uint32_t cnt[9][kMaxSeg + 3];
-  uint32_t dst[27], lead[27], n[27], alen[27];
-  uint32_t src[27];    // mirror slot of each run's first (16-byte aligned) slot
-  float shift[27][3];  // frame shift of each run
-};
-
-// Slots of a stage buffer for `cap` staged atoms: each of up to 3 copy runs
-// per column brings at most 6 neighbouring atoms, plus one quad of far atoms
-// that pads the last chunk of every quad table.
+// Slots of a stage for `cap` staged atoms: every column rounds up to whole
+// blocks, and one block of far atoms pads the block tables.  A multiple of 16,
+// which keeps every part of the shared memory below on a 16-byte boundary.
 __host__ __device__ __forceinline__ uint32_t padded_slots(uint32_t cap) {
-  return ((cap + 162u + 3u) & ~3u) + 4u;
+  return ((cap + 15u) & ~15u) + 9u * 8u + 8u;
 }
+static_assert(warp_bytes(1) % 16 == 0 && warp_bytes(2) % 16 == 0, "tables are read 16 bytes at a time");
 
-__host__ __device__ __forceinline__ uint32_t plane_bytes(uint32_t slots, int nt) {
-  return (slots * (nt > 1 ? 16u : 12u) + 15u) & ~15u;
-}
+// Bytes per slot of the type indicators, and of everything: exact position,
+// fp16 record, type indicators, and a share of the block's z range.
+__host__ __device__ constexpr uint32_t type_bytes(int nt) { return nt > 2 ? 8u : (nt > 1 ? 4u : 0u); }
+__host__ __device__ constexpr uint32_t slot_bytes(int nt) { return 25u + type_bytes(nt); }
 
-// Bytes of one consumer warp's pair lists plus its quad table.
-__host__ __device__ __forceinline__ uint32_t warp_bytes(uint32_t slots) {
-  return ((32u * kListLen * 2u + (slots / 4u + kChunk) * 2u) + 15u) & ~15u;
-}
-
-// Dynamic shared memory of one CTA: two stage buffers and the consumers' lists.
-__host__ __device__ __forceinline__ uint32_t smem_bytes(uint32_t cap, int consumers, int nt) {
-  const uint32_t slots = padded_slots(cap);
-  return 2u * plane_bytes(slots, nt) + (uint32_t)consumers * warp_bytes(slots);
+// Dynamic shared memory of one CTA: the stage, and the warps' tables and lists.
+__host__ __device__ __forceinline__ uint32_t smem_bytes(uint32_t cap, int warps, int nt) {
+  return padded_slots(cap) * slot_bytes(nt) + (uint32_t)warps * warp_bytes(nt);
 }
 
 // MODE kModeCapped: relaxation force of the steepest-descent path, with the
@@ -161,13 +166,9 @@ struct PairAcc {
   }
 };
 
-// Packed accumulators of the phase-2 fast path (FP32 sums, LJ or capped law):
-// each lane keeps two partial sums per quantity, one per list-entry parity.
-template <bool ENERGY>
-struct PairAcc2 {
+// Packed force sums of phase 2 (FP32): one half per home atom of the lane.
+struct Force2 {
   float2 fx = {0.f, 0.f}, fy = {0.f, 0.f}, fz = {0.f, 0.f};
-  float2 pe = {0.f, 0.f}, pes = {0.f, 0.f}, vir = {0.f, 0.f};
-  uint32_t n = 0;
 };
 
 // Global-memory path (stage overflow): lanes are 32 consecutive home atoms,
@@ -187,734 +188,552 @@ __device__ __forceinline__ void global_range(const float4 *__restrict__ P, uint3
   }
 }
 
-// Phase 2, general form: one listed pair per step, any force law and any
-// accumulator type.  Entries are padded slots; the exact cutoff drops the
-// candidates phase 1 admitted through its margin and the self pair.
-template <int NT, bool ENERGY, typename Acc, int MODE>
-__device__ __forceinline__ void flush_scalar(const float *X, const float *Y, const float *Z,
-                                             const uint32_t *T, const uint16_t *list,
-                                             uint32_t cnt, int lane, float xi, float yi, float zi,
-                                             int ti, const LJLocal<NT> &lj,
-                                             PairAcc<NT, ENERGY, Acc, MODE> &a) {
-  for (uint32_t k = 0; k < cnt; ++k) {
-    const uint32_t j = list[k * 32 + lane];
-    const float dx = xi - X[j], dy = yi - Y[j], dz = zi - Z[j];
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-    const int kk = NT == 1 ? 0 : ti * NT + (int)T[j];
-    if (r2 < lj.rc2[kk] && r2 > 0.0f) a.add(lj, kk, dx, dy, dz, r2);
+
+// 0 < r2 < rc2 by one unsigned comparison: floats that are not negative order
+// as their bits, r2 = 0 wraps to the largest value and NaNs lie above every rc2.
+__device__ __forceinline__ bool inside(float r2, uint32_t rc2_less_1) {
+  return __float_as_uint(r2) - 1u < rc2_less_1;
+}
+
+__device__ __forceinline__ uint32_t less_1(float rc2) { return __float_as_uint(rc2) - 1u; }
+
+// D = A B + C of one m16n8k8 product, fp16 operands and FP32 sums.
+__device__ __forceinline__ void mma_16x8x8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b,
+                                           const float (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+      "{%7, %8, %9, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(b), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+
+__device__ __forceinline__ uint4 lds_u4(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
+}
+
+// Stage reads: the stage is read-only once handed over, so the compiler may
+// schedule them freely.
+__device__ __forceinline__ uint32_t lds_stage(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+
+__device__ __forceinline__ uint32_t pack_half2(float lo, float hi) {
+  const __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+__device__ __forceinline__ float2 unpack_half2(uint32_t u) {
+  return __half22float2(*reinterpret_cast<const __half2 *>(&u));
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// LJ tables of the item's system (one warp).
+template <int NT, int MODE>
+__device__ __forceinline__ void load_lj(const ForceBufs &b, const SysDesc &S, Stage<NT> &d) {
+  const LJTable &T = b.lj[S.lj];
+  const float sc = 1.0f / fmaxf(fmaxf(S.g.len[0], S.g.len[1]), S.g.len[2]);
+  const int lane = threadIdx.x & 31;
+  const float most = MODE == kModeSoftCore ? b.sc_rc * b.sc_rc : kFar;
+  float rc2max = 0.f;
+  for (int t = lane; t < NT * NT; t += 32) {
+    const int k = t / NT * T.nt + t % NT;
+    const float rc2 = fminf(T.rc2[k], most);
+    d.lj.s2[t] = T.s2[k];
+    d.lj.e24[t] = T.e24[k];
+    d.lj.e4[t] = T.e4[k];
+    d.lj.rc2[t] = rc2;
+    d.lj.ush[t] = T.ushift[k];
+    if (NT > 1)
+      d.lj4[t] = make_float4(T.s2[k], T.e24[k], __uint_as_float(less_1(rc2)), 0.f);
+    rc2max = fmaxf(rc2max, rc2);
+  }
+  // non-negative floats order as their bits
+  rc2max = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(rc2max)));
+  if (NT > 1 && lane < NT) {
+    float c[4];
+    for (int k = 0; k < 4; ++k) {
+      const float rc2 = k < T.nt && lane < T.nt ? fminf(T.rc2[lane * T.nt + k], most) : rc2max;
+      // rounded down, so that no pair inside its cutoff is lost
+      c[k] = (rc2max - rc2) * sc * sc * (1.0f - 1.0f / 512.0f);
+    }
+    d.cut[lane] = make_uint2(pack_half2(c[0], c[1]), pack_half2(c[2], c[3]));
+  }
+  if (lane == 0) {
+    d.lj.sc_rc = b.sc_rc;
+    d.lj.sc_f0 = b.sc_f0;
+    d.rcw = sqrtf(rc2max) * 1.00001f + 1e-5f;
+    d.rs2 = rc2max * sc * sc;
   }
 }
 
-// Phase 2, fast form (FP32 sums, LJ or capped law): two list entries per step
-// in packed FP32x2 arithmetic; the force of an entry outside the exact cutoff
-// (or past the lane's count) is selected to zero.
-template <int NT, bool ENERGY, int MODE>
-__device__ __forceinline__ void flush_packed(const float *X, const float *Y, const float *Z,
-                                             const uint32_t *T, const uint16_t *list,
-                                             uint32_t cnt, int lane, float xi, float yi, float zi,
-                                             int ti, const LJLocal<NT> &lj,
-                                             PairAcc2<ENERGY> &a) {
-  const float2 m1 = make_float2(-1.0f, -1.0f);
-  const float2 xi2 = make_float2(xi, xi), yi2 = make_float2(yi, yi), zi2 = make_float2(zi, zi);
-  const float2 two = make_float2(2.0f, 2.0f), mone = make_float2(-1.0f, -1.0f);
-  const float2 half = make_float2(0.5f, 0.5f);
-  float2 s2 = make_float2(lj.s2[0], lj.s2[0]), e24 = make_float2(lj.e24[0], lj.e24[0]);
-  float2 e4 = make_float2(lj.e4[0], lj.e4[0]), ush = make_float2(lj.ush[0], lj.ush[0]);
-  float rc2a = lj.rc2[0], rc2b = lj.rc2[0];
-  // shared-memory byte addresses of the planes and of this lane's entries
-  const uint32_t xa = smem_u32(X), ya = smem_u32(Y), za = smem_u32(Z);
-  const uint32_t la = smem_u32(list) + 2u * (uint32_t)lane;
-  for (uint32_t k = 0; k < cnt; k += 2) {
-    const uint32_t j0 = lds_u16(la + 64u * k);
-    const uint32_t j1 = lds_u16(la + 64u * min(k + 1, cnt - 1));
-    const bool v1 = k + 1 < cnt;
-    if (NT > 1) {
-      const int ka = ti * NT + (int)T[j0], kb = ti * NT + (int)T[j1];
-      s2 = make_float2(lj.s2[ka], lj.s2[kb]);
-      e24 = make_float2(lj.e24[ka], lj.e24[kb]);
-      rc2a = lj.rc2[ka];
-      rc2b = lj.rc2[kb];
-      if (ENERGY) {
-        e4 = make_float2(lj.e4[ka], lj.e4[kb]);
-        ush = make_float2(lj.ush[ka], lj.ush[kb]);
+// Lays out the stage of work item `it` and starts its copies (one warp): runs
+// of the sorted positions go to their slots by bulk copies that complete on
+// `full`, and far atoms pad the columns.
+template <int NT>
+__device__ __forceinline__ void plan_stage(const ForceBufs &b, const ForceItem &it, Stage<NT> &d,
+                                           float4 *E, uint64_t *full) {
+  const int lane = threadIdx.x & 31;
+  const SysDesc &S = b.sys[it.sys];
+  const int z0 = it.z0, z1 = it.z1, nz = S.g.n[2];
+  const bool per = S.g.periodic != 0;
+  uint32_t nl = 0, nm = 0, nh = 0, gl = 0, gm = 0, gh = 0, home0 = 0, home1 = 0;
+  if (lane < 9) {
+    const uint32_t kb = it.kbase[lane];
+    d.kbase[lane] = kb;
+    if (per || kb != kNoCell) {  // no column past an open face
+      // the z cells of a column are consecutive keys: its staged cells are one
+      // run, plus an image of the top (bottom) cell below (above) it
+      const uint32_t zl = (uint32_t)max(z0 - 1, 0), zh = (uint32_t)min(z1 + 1, nz);
+      gm = b.start[kb + zl];
+      nm = b.start[kb + zh] - gm;
+      if (per && z0 == 0) {
+        gl = b.start[kb + nz - 1];
+        nl = b.start[kb + nz] - gl;
+      }
+      if (per && z1 == nz) {
+        gh = b.start[kb];
+        nh = b.start[kb + 1] - gh;
+      }
+      if (lane == 4) {
+        home0 = b.start[kb + z0];
+        home1 = b.start[kb + z1];
       }
     }
-    const float2 dx =
-        __ffma2_rn(make_float2(lds_f32(xa + 4u * j0), lds_f32(xa + 4u * j1)), m1, xi2);
-    const float2 dy =
-        __ffma2_rn(make_float2(lds_f32(ya + 4u * j0), lds_f32(ya + 4u * j1)), m1, yi2);
-    const float2 dz =
-        __ffma2_rn(make_float2(lds_f32(za + 4u * j0), lds_f32(za + 4u * j1)), m1, zi2);
-    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    const bool ina = r2.x < rc2a && r2.x > 0.0f;
-    const bool inb = v1 && r2.y < rc2b && r2.y > 0.0f;
-    float2 r2c = r2;
-    if (MODE == kModeCapped) {
-      const float2 fl = __fmul2_rn(make_float2(0.25f, 0.25f), s2);
-      r2c = make_float2(fmaxf(r2.x, fl.x), fmaxf(r2.y, fl.y));
+  }
+  const uint32_t n = nl + nm + nh, slots = (n + 7u) & ~7u;
+  uint32_t incl = slots, atoms = n;
+#pragma unroll
+  for (int o = 1; o < 16; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+    atoms += __shfl_xor_sync(0xffffffffu, atoms, o);
+  }
+  const uint32_t first = incl - slots;
+  const uint32_t total = __shfl_sync(0xffffffffu, incl, 8);
+  // the system's own capacity decides: the same path alone or batched
+  const uint32_t H = __shfl_sync(0xffffffffu, home1 - home0, 4);
+  const uint32_t ntile = (H + kTile - 1) / kTile;
+  const bool overflow = total + 8u > padded_slots(S.cap) || ntile > (uint32_t)kWinCap;
+  const bool copy = !overflow && !(b.test_flags & 1u);  // test hook: the copies never arrive
+  if (copy && lane == 0) mbar_arrive_expect_tx(full, 16u * atoms);
+  __syncwarp();
+  if (lane < 9) {
+    if (copy) {
+      if (nl) bulk_g2s(E + first, b.rs + gl, 16u * nl, full);
+      if (nm) bulk_g2s(E + first + nl, b.rs + gm, 16u * nm, full);
+      if (nh) bulk_g2s(E + first + nl + nm, b.rs + gh, 16u * nh, full);
+      for (uint32_t k = first + n; k < first + slots; ++k)
+        E[k] = make_float4(kFar, kFar, kFar, 0.f);
     }
-    const float2 inv = make_float2(rcp_approx(r2c.x), rcp_approx(r2c.y));
-    const float2 sr2 = __fmul2_rn(s2, inv);
-    const float2 sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
-    const float2 t = __ffma2_rn(two, sr6, mone);
-    float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(e24, sr6), t), inv);
-    f.x = ina ? f.x : 0.0f;
-    f.y = inb ? f.y : 0.0f;
-    a.fx = __ffma2_rn(f, dx, a.fx);
-    a.fy = __ffma2_rn(f, dy, a.fy);
-    a.fz = __ffma2_rn(f, dz, a.fz);
-    if (ENERGY) {
-      float2 u = __fmul2_rn(__fmul2_rn(e4, sr6), __fadd2_rn(sr6, mone));
-      u.x = ina ? u.x : 0.0f;
-      u.y = inb ? u.y : 0.0f;
-      float2 us = __fadd2_rn(u, make_float2(-ush.x, -ush.y));
-      us.x = ina ? us.x : 0.0f;
-      us.y = inb ? us.y : 0.0f;
-      a.pe = __ffma2_rn(half, u, a.pe);
-      a.pes = __ffma2_rn(half, us, a.pes);
-      a.vir = __ffma2_rn(__fmul2_rn(half, f), r2c, a.vir);
-      a.n += (uint32_t)ina + (uint32_t)inb;
+    d.c0[lane] = first;
+    d.e0[lane] = first + nl;
+    d.e1[lane] = first + nl + nm;
+    d.e2[lane] = first + n;
+  } else if (copy && lane < 17) {
+    E[total + (uint32_t)lane - 9u] = make_float4(kFar, kFar, kFar, 0.f);
+  }
+  if (lane == 4) {
+    d.c0[9] = total;
+    d.home_g0 = home0;
+    d.H = H;
+    d.hb = first + nl + (home0 - gm);
+    d.ntile = ntile;
+    d.overflow = overflow;
+    if (overflow) {
+      d.ntile = min((H + 31) / 32, (uint32_t)kWinCap);
+      atomicOr(&b.status[it.sys], kStatusSmemOverflow);
     }
   }
 }
 
-// ---- producer ---------------------------------------------------------------
-
-// Set up item `item` in descriptor `d` and stage buffer `pl` (the kProd
-// producer warps together).  Returns false when the wait for the bulk copies
-// gave up.
-template <int NT, int MODE, int kProd, int kCons>
-__device__ bool produce_item(const ForceBufs &b, uint32_t item, ItemDesc<NT> &d, Scratch &sc,
-                             const Planes &pl, uint32_t &running) {
-  constexpr int kPT = kProd * 32;  // producer threads
-  const int pt = threadIdx.x, lane = pt & 31, pw = pt >> 5;
-  const ForceItem it = b.items[item];
-  const bool skip = b.steps_left != nullptr && b.steps_left[it.sys] == 0;
-  if (pt == 0) {
-    d.item = item;
-    d.sys = it.sys;
-    d.skip = skip;
-    d.overflow = 0;
-    d.H = 0;
-    d.nclus = 0;
-    d.ntask = 0;
-  }
-  if (skip) {  // a system whose step budget is spent keeps its state
-    producer_sync<kProd>();
-    return true;
-  }
-  const SysDesc &S = b.sys[it.sys];
-  const Grid g = S.g;
-  const uint32_t mirror0 = S.mirror0, atom0 = S.atom0, scap = S.cap;
-  const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-  const int z0 = it.z0, z1 = it.z1, nseg = z1 - z0;
-  const int ncell = nseg + 2;  // staged cells per column
+// Frame shifts and constants of the item (one warp).
+template <int NT>
+__device__ __forceinline__ void plan_frame(const ForceBufs &b, const ForceItem &it, Stage<NT> &d) {
+  const int lane = threadIdx.x & 31;
+  const Grid &g = b.sys[it.sys].g;
+  const int z0 = it.z0, z1 = it.z1, nz = g.n[2];
   const bool per = g.periodic != 0;
-  for (int t = pt; t < NT * NT; t += kPT) {
-    const LJTable &Tb = b.lj[S.lj];
-    const int a = t / NT, c = t % NT;
-    const int k = a * Tb.nt + c;
-    d.lj.s2[t] = Tb.s2[k];
-    d.lj.e24[t] = Tb.e24[k];
-    d.lj.e4[t] = Tb.e4[k];
-    d.lj.rc2[t] = MODE == kModeSoftCore ? fminf(Tb.rc2[k], b.sc_rc * b.sc_rc) : Tb.rc2[k];
-    d.lj.ush[t] = Tb.ushift[k];
-  }
-  if (pt < 9) {
-    const int cx = it.cx, cy = it.cy;
-    const int c = pt;
-    const int ax = cx + c / 3 - 1, ay = cy + c % 3 - 1;
-    const int wx = ax < 0 ? -1 : (ax >= nx ? 1 : 0);
-    const int wy = ay < 0 ? -1 : (ay >= ny ? 1 : 0);
-    // frame: F = L on the top face; staged = x + w L - F, so the shift is F - w L
-    // (an open box has no images and no frame shift)
-    const float Fx = per && cx == nx - 1 ? g.L[0] : 0.0f, Fy = per && cy == ny - 1 ? g.L[1] : 0.0f;
-    d.sx[c] = per ? Fx - (float)wx * g.L[0] : 0.0f;
-    d.sy[c] = per ? Fy - (float)wy * g.L[1] : 0.0f;
-    d.kbase[c] = it.kbase[c];
-  }
   // an item on the top face works in the frame shifted down by L, where the
   // shifts of its atoms (all in the upper half) are exact; a whole column
   // keeps the unshifted frame and rounds only the image above its top
+  const float Fx = per && it.cx == g.n[0] - 1 ? g.L[0] : 0.0f;
+  const float Fy = per && it.cy == g.n[1] - 1 ? g.L[1] : 0.0f;
   const float Fz = per && z1 == nz && z0 > 0 ? g.L[2] : 0.0f;
-  const float sz_lo = per && z0 == 0 ? Fz + g.L[2] : Fz;  // image z0 - 1 wraps below when z0 == 0
-  const float sz_hi = per && z1 == nz ? Fz - g.L[2] : Fz;  // image z1 wraps above when z1 == nz
-  if (pt == 0) {
-    d.sz_lo = sz_lo;
-    d.sz_mid = Fz;
-    d.sz_hi = sz_hi;
+  float sx = 0.f, sy = 0.f;
+  if (lane < 9 && per) {
+    const int ax = it.cx + lane / 3 - 1, ay = it.cy + lane % 3 - 1;
+    const int wx = ax < 0 ? -1 : (ax >= g.n[0] ? 1 : 0);
+    const int wy = ay < 0 ? -1 : (ay >= g.n[1] ? 1 : 0);
+    // frame: F = L on the top face; staged = x + w L - F, so the shift is F - w L
+    // (an open box has no images and no frame shift)
+    sx = Fx - (float)wx * g.L[0];
+    sy = Fy - (float)wy * g.L[1];
+  }
+  if (lane < 9) {
+    d.sx[lane] = sx;
+    d.sy[lane] = sy;
+  }
+  const bool any = __any_sync(0xffffffffu, sx != 0.f || sy != 0.f);
+  if (lane == 0) {
+    d.szm = Fz;
+    d.szl = per ? Fz + g.L[2] : Fz;  // image z0 - 1 wraps below when z0 == 0
+    d.szh = per ? Fz - g.L[2] : Fz;  // image z1 wraps above when z1 == nz
+    d.shifted = any || (per && (z0 == 0 || z1 == nz));
+    d.cx = g.lo[0] + ((float)it.cx + 0.5f) * g.len[0] - Fx;
+    d.cy = g.lo[1] + ((float)it.cy + 0.5f) * g.len[1] - Fy;
+    d.cz = g.lo[2] + 0.5f * (float)(z0 + z1) * g.len[2] - Fz;
+    d.scale = 1.0f / fmaxf(fmaxf(g.len[0], g.len[1]), g.len[2]);
     d.z0 = z0;
     d.nz = nz;
-    d.nseg = nseg;
+    d.nseg = z1 - z0;
     d.periodic = per;
-    d.lj.sc_rc = b.sc_rc;
-    d.lj.sc_f0 = b.sc_f0;
+    d.nmax = 0u;
   }
-  // cell starts and counts of the 9 x ncell staged cells; in an open box a
-  // column past a face, or a cell past the bottom or top, is empty
-  for (int t = pt; t < 9 * ncell; t += kPT) {
-    const int c = t / ncell, k = t % ncell;
-    const int zr = z0 - 1 + k, zc = (zr + nz) % nz;
-    uint32_t s0 = 0, s1 = 0;
-    if (per || (it.kbase[c] != kNoCell && zr >= 0 && zr < nz)) {
-      const uint32_t key = it.kbase[c] + (uint32_t)zc;
-      s0 = b.start[key];
-      s1 = b.start[key + 1];
+}
+
+// Moves the staged atoms into the item's frame, a warp per column (x - 0 is x,
+// so unshifted atoms pass unchanged).
+template <int NT, int kWarps>
+__device__ __forceinline__ void shift_stage(const Stage<NT> &d, float4 *E) {
+  for (int c = threadIdx.x >> 5; c < 9; c += kWarps) {
+    const float sx = d.sx[c], sy = d.sy[c];
+    const uint32_t e0 = d.e0[c], e1 = d.e1[c], e2 = d.e2[c];
+    for (uint32_t u = d.c0[c] + (threadIdx.x & 31); u < e2; u += 32) {
+      float4 q = E[u];
+      q.x -= sx;
+      q.y -= sy;
+      q.z -= u < e0 ? d.szl : (u < e1 ? d.szm : d.szh);
+      E[u] = q;
     }
-    sc.gstart[c][k] = s0;
-    sc.cnt[c][k] = s1 - s0;
   }
-  producer_sync<kProd>();
-  // exclusive prefix over the cells of each column, one warp per column
-  for (int c = pw; c < 9; c += kProd) {
-    uint32_t run = 0;
-    for (int base = 0; base < ncell; base += 32) {
-      const int k = base + lane;
-      const uint32_t v = k < ncell ? sc.cnt[c][k] : 0u;
-      uint32_t incl = v;
+}
+
+// fp16 records and block z ranges of the stage, all threads of the CTA.  An
+// atom with a non-finite coordinate (a simulation that has blown up) becomes a
+// far atom, and makes the z range of its block NaN, which no window excludes.
+// Far atoms have infinite or NaN records: no hit, or one that the exact test
+// drops.
+template <int NT, int kWarps>
+__device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf, uint32_t *Ht, float *zb) {
+  const uint32_t total = d.c0[9];
+  const float cx = d.cx, cy = d.cy, cz = d.cz, sc = d.scale;
+  float nmax = 0.f;
+  for (uint32_t u = threadIdx.x; u < total + 8u; u += kWarps * 32) {
+    const float4 q = E[u];
+    const uint32_t xy = pack_half2((q.x - cx) * sc, (q.y - cy) * sc);
+    const float2 r = unpack_half2(xy);
+    const float zr = (q.z - cz) * sc, z = __half2float(__float2half_rn(zr));
+    const float n = fmaf(r.x, r.x, fmaf(r.y, r.y, z * z));
+    Hf[u] = make_uint2(xy, pack_half2(zr, n));
+    if (NT > 1) {
+      const uint32_t ty = (uint32_t)__float_as_int(q.w), one = ty & 1u ? 0x3c000000u : 0x3c00u;
+      const uint32_t lo = ty < 2u ? one : 0u, hi = ty >= 2u && ty < 4u ? one : 0u;
+      if (NT == 2)
+        Ht[u] = lo;
+      else
+        reinterpret_cast<uint2 *>(Ht)[u] = make_uint2(lo, hi);
+    }
+    const float far = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
+    if (far < 1e29f && !isnan(n))
+      nmax = fmaxf(nmax, n);
+    else
+      E[u] = make_float4(kFar, kFar, kFar, q.w);
+    const uint32_t k = u & 7u;
+    // q.z - q.z is 0, or NaN where z is not finite
+    if (k == 0u || k == 7u) zb[(u >> 3) * 2u + (k >> 2)] = q.z + (q.z - q.z);
+  }
+  const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(nmax));
+  if ((threadIdx.x & 31) == 0) atomicMax(&d.nmax, m);
+}
+
+// One tile of 16 home atoms (one warp); energy sums (pe, shifted pe, virial,
+// pairs) in `ce`.
+template <int NT, bool ENERGY, typename Acc, int MODE>
+__device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> &d,
+                                            const float4 *E, const uint2 *Hf, const uint32_t *Ht,
+                                            const float *zb, uint32_t tile, uint32_t *tab, double *ce) {
+  constexpr bool kPacked = MODE != kModeSoftCore;
+  constexpr bool kSum32 = std::is_same<Acc, float>::value;
+  const int lane = threadIdx.x & 31;
+  const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u;
+  const uint32_t H = d.H, h0 = tile * kTile, hb = d.hb + h0;
+  // home atoms of this lane: rows g and g + 8 of the mma hold the neighbouring
+  // atoms 2 g and 2 g + 1 of the tile, which share most of their candidates
+  const bool va = h0 + 2 * g < H, vb = h0 + 2 * g + 1 < H;
+  const uint32_t sa = hb + (va ? 2 * g : 0u), sb = hb + (vb ? 2 * g + 1 : 0u);
+  float4 pa = E[sa], pb = E[sb];
+  if (!va) pa.x = pa.y = pa.z = kNoAtom;
+  if (!vb) pb.x = pb.y = pb.z = kNoAtom;
+  // the particle index of the force store, fetched now so that its latency
+  // passes during the pair loops (lane t = 0 stores atom a, t = 1 atom b)
+  const uint32_t pi = (t == 0 && va) || (t == 1 && vb)
+                          ? __ldg(b.pid + d.home_g0 + h0 + 2 * g + t) : 0u;
+
+  // operands of the distance product: A rows (-2 x, -2 y, -2 z, 1), C the
+  // rows' squared norm less the bound
+  const uint2 ha = Hf[sa], hbv = Hf[sb];
+  uint32_t a0 = 0u, a1 = 0u;
+  float C[4];
+  {
+    const float2 axy = unpack_half2(ha.x), bxy = unpack_half2(hbv.x);
+    const float az = unpack_half2(ha.y).x, bz = unpack_half2(hbv.y).x;
+    if (t == 0) {
+      a0 = pack_half2(-2.f * axy.x, -2.f * axy.y);
+      a1 = pack_half2(-2.f * bxy.x, -2.f * bxy.y);
+    } else if (t == 1) {
+      a0 = pack_half2(-2.f * az, 1.f);
+      a1 = pack_half2(-2.f * bz, 1.f);
+    } else if (NT > 1) {
+      const uint2 ca = d.cut[__float_as_int(pa.w)], cb = d.cut[__float_as_int(pb.w)];
+      a0 = t == 2 ? ca.x : ca.y;
+      a1 = t == 2 ? cb.x : cb.y;
+    }
+    // bound: rounding a record moves the point by at most 2^-11 of its norm,
+    // and the stored norm by 2^-11 of itself
+    const float nm = __uint_as_float(d.nmax), dl = sqrt_approx(nm) * (1.0f / 1024.0f);
+    const float bound =
+        d.rs2 + 1.05f * (2.0f * sqrt_approx(d.rs2) * dl + dl * dl + nm * (1.0f / 2048.0f)) + 1e-4f;
+    C[0] = C[1] = va ? fmaf(axy.x, axy.x, fmaf(axy.y, axy.y, az * az)) - bound : kFar;
+    C[2] = C[3] = vb ? fmaf(bxy.x, bxy.x, fmaf(bxy.y, bxy.y, bz * bz)) - bound : kFar;
+  }
+  const uint32_t eb = smem_u32(E) + 32u * t;  // candidate 2 t of a block
+  // B operand: candidate g; lanes t >= 2 hold its type indicators (one type:
+  // their A operand is zero, and they repeat the record)
+  const bool types = NT > 1 && t >= 2;
+  const uint32_t stride = types ? type_bytes(NT) : 8u;
+  const uint32_t hbase = (types ? smem_u32(Ht) : smem_u32(Hf)) + stride * g +
+                         (stride == 8u ? 4u * (t & 1u) : 0u);
+  const uint32_t tb = smem_u32(tab);
+  const uint32_t lbase = tb + kTabBytes + 2u * (uint32_t)lane;   // this lane's list, entry k at + 64 k
+  const uint32_t far = d.c0[9];
+
+  PairAcc<NT, ENERGY, Acc, MODE> acca, accb;
+  Force2 acc;
+  const float2 m1 = make_float2(-1.0f, -1.0f);
+  const int ta = NT == 1 ? 0 : __float_as_int(pa.w) * NT;
+  const int tbt = NT == 1 ? 0 : __float_as_int(pb.w) * NT;
+  float2 s2 = make_float2(d.lj.s2[0], d.lj.s2[0]);
+  float2 e24 = make_float2(d.lj.e24[0], d.lj.e24[0]);
+  uint32_t rca = less_1(d.lj.rc2[0]), rcb = rca;  // bits of rc^2, less one
+  float4 l0a, l1a, l0b, l1b;
+  if (NT == 2) {
+    l0a = d.lj4[ta];
+    l1a = d.lj4[ta + 1];
+    l0b = d.lj4[tbt];
+    l1b = d.lj4[tbt + 1];
+  }
+
+  // the tile's z window (all z when its first atom is a far one)
+  const float z0 = E[hb].z, z1 = E[hb + min((uint32_t)kTile, H - h0) - 1].z;
+  const float zlo = z0 < 1e29f ? z0 - d.rcw : -kFar, zhi = z1 + d.rcw;
+  const uint32_t blocks = d.c0[9] >> 3;
+  for (uint32_t blk = 0; blk < blocks;) {
+    // table: first slots of the blocks in the window; far blocks pad it to a
+    // multiple of 4
+    __syncwarp();
+    uint32_t nt = 0;
+    for (; blk < blocks && nt <= (uint32_t)kTabBlocks - 36u; blk += 32) {
+      const uint32_t i = blk + (uint32_t)lane;
+      const float2 z = reinterpret_cast<const float2 *>(zb)[min(i, blocks)];
+      const bool in = i < blocks && !(z.y < zlo) && !(z.x > zhi);
+      const uint32_t m = __ballot_sync(0xffffffffu, in);
+      if (in) tab[nt + __popc(m & ((1u << lane) - 1u))] = 8u * i;
+      nt += __popc(m);
+    }
+    const uint32_t cb4 = (nt + 3u) & ~3u;
+    if (lane < 4 && nt + lane < cb4) tab[nt + lane] = far;
+    __syncwarp();
+    uint32_t u = 0;
+    do {
+      // phase 1: until all blocks are tested or some lane's list is nearly full
+      uint32_t oa = lbase;
+      for (; u < cb4; u += 4) {
+        if (__any_sync(0xffffffffu, oa > lbase + 64u * (list_len(NT) - 8u))) break;
+        const uint4 o4 = lds_u4(tb + 4u * u);
+        const uint32_t o[4] = {o4.x, o4.y, o4.z, o4.w};
+        uint32_t B[4];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      if (k < ncell) d.off[c][k] = run + incl - v;
-      run += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (lane == 0) d.off[c][ncell] = run;
-  }
-  producer_sync<kProd>();
-  // copy runs: piece 0 = image cell z0 - 1 when z0 == 0, piece 2 = image cell
-  // z1 when z1 == nz, piece 1 = the cells between (consecutive z, one run)
-  const int a_end = z0 == 0 ? 1 : 0, c_beg = z1 == nz ? ncell - 1 : ncell;
-  const uint32_t H = d.off[4][nseg + 1] - d.off[4][1];
-  const uint32_t nclus = (H + 7) / 8;
-  if (pw == 0) {
-    uint32_t n = 0, m0 = 0, ma = 0, alen = 0;
-    if (lane < 27) {
-      const int c = lane / 3, p = lane % 3;
-      const int k0 = p == 0 ? 0 : (p == 1 ? a_end : c_beg);
-      const int k1 = p == 0 ? a_end : (p == 1 ? c_beg : ncell);
-      n = d.off[c][k1] - d.off[c][k0];
-      if (n > 0) {
-        m0 = mirror0 + (sc.gstart[c][k0] - atom0);
-        ma = m0 & ~3u;
-        alen = ((m0 + n + 3u) & ~3u) - ma;
-      }
-    }
-    uint32_t incl = alen;
+        for (int j = 0; j < 4; ++j) B[j] = lds_stage(hbase + (NT == 2 ? stride : 8u) * o[j]);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    const uint32_t dst = incl - alen;
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    // frame shift of each run: the column's x, y shift and the run's z shift
-    float rx = 0.f, ry = 0.f, rz = 0.f;
-    if (lane < 27) {
-      const int c = lane / 3, pp = lane % 3;
-      rx = d.sx[c];
-      ry = d.sy[c];
-      rz = pp == 0 ? sz_lo : (pp == 1 ? Fz : sz_hi);
-      sc.dst[lane] = dst;
-      sc.src[lane] = ma;
-      sc.lead[lane] = m0 - ma;
-      sc.n[lane] = n;
-      sc.alen[lane] = alen;
-      sc.shift[lane][0] = rx;
-      sc.shift[lane][1] = ry;
-      sc.shift[lane][2] = rz;
-      if (lane % 3 == 0) d.ps[lane / 3] = dst;
-    }
-    // the system's own capacity decides: the same path alone or batched
-    const bool overflow = total + 4u > padded_slots(scap) || nclus > (uint32_t)kWinCap;
-    if (lane == 0) {
-      d.ps[9] = total;
-      d.H = H;
-      d.home_g0 = sc.gstart[4][1];
-      d.overflow = overflow;
-      if (overflow) {
-        d.ntask = min((H + 31) / 32, (uint32_t)kWinCap);
-        atomicOr(&b.status[it.sys], kStatusSmemOverflow);
-      }
-    }
-  }
-  producer_sync<kProd>();
-  if (d.overflow) return true;
-  const uint32_t total = d.ps[9];
-  if (total > 0) {
-    // the runs' 16-byte quads, all producer threads, each run moved into the
-    // item's frame on the way (x - 0 is x, so unshifted runs pass unchanged);
-    // kCopyBatch quads per thread are loaded before any is stored
-    constexpr int kB = NT > 1 ? kCopyBatch / 2 : kCopyBatch;  // the type plane takes registers
-    const uint32_t nq = total >> 2;
-    int p = 0;
-    for (uint32_t u0 = pt; u0 < nq; u0 += kB * kPT) {
-      float4 vx[kB], vy[kB], vz[kB];
-      uint4 vt[NT > 1 ? kB : 1];
-      int pr[kB];
-#pragma unroll
-      for (int k = 0; k < kB; ++k) {
-        const uint32_t u = u0 + (uint32_t)k * kPT;
-        pr[k] = -1;
-        if (u < nq) {
-          while (4u * u >= sc.dst[p] + sc.alen[p]) ++p;  // runs in slot order
-          pr[k] = p;
-          const uint32_t g = sc.src[p] + (4u * u - sc.dst[p]);
-          vx[k] = ldg_f4(b.xs + g);
-          vy[k] = ldg_f4(b.ys + g);
-          vz[k] = ldg_f4(b.zs + g);
-          if (NT > 1) vt[k] = ldg_u4(b.ts + g);
+        for (int j = 0; j < 4; ++j) {
+          float D[4];
+          mma_16x8x8(D, a0, a1, B[j], C);
+          if ((__float_as_uint(D[0]) | __float_as_uint(D[2])) & 0x80000000u) {
+            sts_u16(oa, o[j]);
+            oa += 64u;
+          }
+          if ((__float_as_uint(D[1]) | __float_as_uint(D[3])) & 0x80000000u) {
+            sts_u16(oa, o[j] + 1u);
+            oa += 64u;
+          }
         }
       }
-#pragma unroll
-      for (int k = 0; k < kB; ++k) {
-        if (pr[k] < 0) break;
-        const uint32_t s = 4u * (u0 + (uint32_t)k * kPT);
-        const float sx = sc.shift[pr[k]][0], sy = sc.shift[pr[k]][1], sz = sc.shift[pr[k]][2];
-        sts_f4(smem_u32(pl.X + s), make_float4(vx[k].x - sx, vx[k].y - sx, vx[k].z - sx, vx[k].w - sx));
-        sts_f4(smem_u32(pl.Y + s), make_float4(vy[k].x - sy, vy[k].y - sy, vy[k].z - sy, vy[k].w - sy));
-        sts_f4(smem_u32(pl.Z + s), make_float4(vz[k].x - sz, vz[k].y - sz, vz[k].z - sz, vz[k].w - sz));
-        if (NT > 1) *reinterpret_cast<uint4 *>(pl.T + s) = vt[k];
-      }
-    }
-    producer_sync<kProd>();
-    // neighbouring atoms that rode along become far atoms that keep z sorted
-    if (pt < 27 && sc.alen[pt] > 0) {
-      const uint32_t dst = sc.dst[pt], s0 = dst + sc.lead[pt], s1 = s0 + sc.n[pt];
-      const float zlo = pl.Z[s0], zhi = pl.Z[s1 - 1];
-      for (uint32_t s = dst; s < s0; ++s) {
-        pl.X[s] = kFar;
-        pl.Y[s] = kFar;
-        pl.Z[s] = zlo;
-        if (NT > 1) pl.T[s] = 0u;
-      }
-      for (uint32_t s = s1; s < dst + sc.alen[pt]; ++s) {
-        pl.X[s] = kFar;
-        pl.Y[s] = kFar;
-        pl.Z[s] = zhi;
-        if (NT > 1) pl.T[s] = 0u;
-      }
-    }
-  }
-  if (pt >= 32 * (kProd - 1) && pt < 32 * (kProd - 1) + 4) {
-    // the quad of far atoms that pads the last chunk of a table
-    const uint32_t s = total + (uint32_t)(pt - 32 * (kProd - 1));
-    pl.X[s] = kFar;
-    pl.Y[s] = kFar;
-    pl.Z[s] = kFar;
-    if (NT > 1) pl.T[s] = 0u;
-  }
-  producer_sync<kProd>();
-  // z windows of every (cluster, column)
-  const int hp = 4 * 3 + 1;  // the home column's middle run holds home cells 1..nseg
-  const uint32_t hb = sc.dst[hp] + sc.lead[hp] + (d.off[4][1] - d.off[4][a_end]);
-  float rcmax2 = 0.f;
-  for (int k = 0; k < NT * NT; ++k) rcmax2 = fmaxf(rcmax2, d.lj.rc2[k]);
-  const float rcw = sqrtf(rcmax2) * 1.00001f + 1e-5f;
-  for (uint32_t t = pt; t < 9u * nclus; t += kPT) {
-    const uint32_t k = t / 9u, c = t - 9u * k;
-    const float zmin = pl.Z[hb + k * 8];
-    const float zmax = pl.Z[hb + min(k * 8 + 7, H - 1)];
-    const uint32_t lo = d.ps[c], hi = d.ps[c + 1];
-    const uint32_t a = lower_bound_z(pl.Z, lo, hi, zmin - rcw) >> 2;
-    const uint32_t e = (upper_bound_z(pl.Z, lo, hi, zmax + rcw) + 3u) >> 2;
-    d.q0[k][c] = (uint16_t)a;
-    // empty unless ordered (an unsorted column, e.g. NaN positions, can
-    // invert the two searches)
-    d.len[k][c] = (uint16_t)(e > a ? e - a : 0u);
-  }
-  producer_sync<kProd>();
-  for (uint32_t k = pt; k < nclus; k += kPT) {
-    uint32_t s = 0, m = 2;
-    for (int c = 0; c < 9; ++c) {
-      d.pre[k][c] = (uint16_t)s;
-      s += d.len[k][c];
-      m = max(m, (uint32_t)d.len[k][c]);
-    }
-    d.Q[k] = (uint16_t)s;
-    d.M[k] = (uint16_t)m;
-  }
-  if (pt == 0) {
-    d.hb = hb;
-    d.nclus = nclus;
-    d.sentinel = total / 4u;
-    d.base = running % (uint32_t)kCons;
-  }
-  running += nclus;
-  producer_sync<kProd>();
-  return true;
-}
-
-// Energy partials of a finished item: its per-cluster (or per-task) sums in
-// cluster order.
-template <int NT>
-__device__ void write_partials(const ForceBufs &b, const ItemDesc<NT> &d, const double (*e)[4]) {
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  if (!d.skip) {
-    const uint32_t n = d.overflow ? d.ntask : d.nclus;
-    for (uint32_t k = 0; k < n; ++k) {
-      v[0] += e[k][0];
-      v[1] += e[k][1];
-      v[2] += e[k][2];
-      v[3] += e[k][3];
-    }
-  }
-  for (int k = 0; k < 4; ++k) b.partials[(size_t)d.item * 4 + k] = v[k];
-}
-
-// ---- consumers --------------------------------------------------------------
-
-// One cluster of 8 home atoms (consumer warp, all 32 lanes); returns the
-// cluster's energy sums in lane 0 (pe, shifted pe, virial, pairs).
-template <int NT, bool ENERGY, typename Acc, int MODE>
-__device__ __forceinline__ void consume_cluster(const ForceBufs &b, const ItemDesc<NT> &d,
-                                                const Planes &pl, uint32_t cl, uint16_t *mylist,
-                                                uint16_t *tb, double (&ce)[4]) {
-  constexpr bool kPacked = std::is_same<Acc, float>::value && MODE != kModeSoftCore;
-  const int lane = threadIdx.x & 31;
-  const int il = lane & 7, q = lane >> 3;
-  const float *X = pl.X, *Y = pl.Y, *Z = pl.Z;
-  const uint32_t *T = pl.T;
-  const uint32_t H = d.H, hb = d.hb;
-  const uint32_t h = cl * 8 + il;
-  const bool valid = h < H;
-  const uint32_t hs = hb + (valid ? h : H - 1);
-  const float xi = valid ? X[hs] : kNoAtom;
-  const float yi = valid ? Y[hs] : kNoAtom;
-  const float zi = valid ? Z[hs] : kNoAtom;
-  // the particle index of the force store, fetched now so that its latency
-  // passes during the pair loops
-  const uint32_t pi = valid && q == 0 ? __ldg(b.pid + d.home_g0 + h) : 0u;
-  const int ti = NT == 1 ? 0 : (int)T[hs];
-  // the warp's quad table: lanes cover (column, index) pairs, column = idx / M
-  // by a multiply-high (exact while 9 M^2 < 2^32)
-  const uint32_t Q = d.Q[cl], M = d.M[cl];
-  const uint32_t magic = 0xffffffffu / M + 1u;
-  for (uint32_t idx = lane; idx < 9u * M; idx += 32) {
-    const uint32_t c = __umulhi(idx, magic), i = idx - c * M;
-    if (i < d.len[cl][c]) tb[table_pos(d.pre[cl][c] + i)] = (uint16_t)(d.q0[cl][c] + i);
-  }
-  for (uint32_t u = Q + lane; u < ((Q + 15u) & ~15u); u += 32)
-    tb[table_pos(u)] = (uint16_t)d.sentinel;
-  __syncwarp();
-
-  float rcmax2 = 0.f;
-  for (int k = 0; k < NT * NT; ++k) rcmax2 = fmaxf(rcmax2, d.lj.rc2[k]);
-  // phase-1 bound with a margin: a superset of the exact test of phase 2
-  const float2 nrc = make_float2(-rcmax2 * (1.0f + 1.0f / 1024.0f),
-                                 -rcmax2 * (1.0f + 1.0f / 1024.0f));
-  const float2 m1 = make_float2(-1.0f, -1.0f);
-  PairAcc<NT, ENERGY, Acc, MODE> acc;
-  PairAcc2<ENERGY> acc2;
-  auto flush = [&](uint32_t cnt) {
-    if constexpr (kPacked) {
-      flush_packed<NT, ENERGY, MODE>(X, Y, Z, T, mylist, cnt, lane, xi, yi, zi, ti, d.lj, acc2);
-    } else {
-      flush_scalar<NT, ENERGY, Acc, MODE>(X, Y, Z, T, mylist, cnt, lane, xi, yi, zi, ti, d.lj,
-                                          acc);
-    }
-  };
-  const float2 xi2 = make_float2(xi, xi), yi2 = make_float2(yi, yi), zi2 = make_float2(zi, zi);
-  // shared-memory byte addresses: candidate planes, and this lane's list
-  // entries at lbase + 64 k (entry k of lane `lane`)
-  const uint32_t xa = smem_u32(X), ya = smem_u32(Y), za = smem_u32(Z);
-  const uint32_t lbase = smem_u32(mylist) + 2u * (uint32_t)lane;
-  uint32_t oa = lbase;  // shared-memory address of this lane's next list entry
-  // lane q tests quads u = q, q + 4, ... of the flat sequence, 4 per chunk; the
-  // table pads the last chunk with the quad of far atoms
-  for (uint32_t u0 = 0; u0 < Q; u0 += kChunk) {
-    const uint32_t cnt = (oa - lbase) >> 6;
-    if (__reduce_max_sync(0xffffffffu, cnt) > (uint32_t)(kListLen - kChunk)) {
-      flush(cnt);
       __syncwarp();
-      oa = lbase;
-    }
-    const uint2 qq = *reinterpret_cast<const uint2 *>(tb + u0 + 4 * q);
-    const uint32_t quads[4] = {qq.x & 0xffffu, qq.x >> 16, qq.y & 0xffffu, qq.y >> 16};
-    // steps of this chunk that hold a real quad for some lane (warp-uniform)
-    const uint32_t nsteps = min((Q - u0 + 3u) >> 2, (uint32_t)(kChunk / 4));
-    // one quad: 4 candidate tests, appended through offsets that depend on
-    // the hit bits only, so the list pointer carries one add per quad
-    auto test_quad = [&](uint32_t quad) {
-      const float4 x4 = lds_f4(xa + quad * 16u), y4 = lds_f4(ya + quad * 16u),
-                   z4 = lds_f4(za + quad * 16u);
-      const float2 dxa = __ffma2_rn(make_float2(x4.x, x4.y), m1, xi2);
-      const float2 dxb = __ffma2_rn(make_float2(x4.z, x4.w), m1, xi2);
-      const float2 dya = __ffma2_rn(make_float2(y4.x, y4.y), m1, yi2);
-      const float2 dyb = __ffma2_rn(make_float2(y4.z, y4.w), m1, yi2);
-      const float2 dza = __ffma2_rn(make_float2(z4.x, z4.y), m1, zi2);
-      const float2 dzb = __ffma2_rn(make_float2(z4.z, z4.w), m1, zi2);
-      const float2 da = __ffma2_rn(dza, dza, __ffma2_rn(dya, dya, __ffma2_rn(dxa, dxa, nrc)));
-      const float2 db = __ffma2_rn(dzb, dzb, __ffma2_rn(dyb, dyb, __ffma2_rn(dxb, dxb, nrc)));
-      // hit = sign bit of r^2 - rc^2 (1 + 2^-10); a -0 or NaN sign only admits a
-      // candidate that phase 2's exact test then drops
-      const uint32_t h0 = __float_as_uint(da.x) >> 31, h1 = __float_as_uint(da.y) >> 31;
-      const uint32_t h2 = __float_as_uint(db.x) >> 31, h3 = __float_as_uint(db.y) >> 31;
-      const uint32_t c1 = h0, c2 = h0 + h1, c3 = c2 + h2, c4 = c3 + h3;
-      // the stores are in bounds whether or not they are kept: the check above
-      // leaves room for every candidate of this chunk
-      const uint32_t s = quad * 4u;
-      sts_u16(oa, s);
-      sts_u16(oa + 64u * c1, s + 1u);
-      sts_u16(oa + 64u * c2, s + 2u);
-      sts_u16(oa + 64u * c3, s + 3u);
-      oa += 64u * c4;
-    };
-    if (nsteps == (uint32_t)(kChunk / 4)) {
+      // phase 2: the exact pairs of every hit; a lane past its last one takes a far atom
+      // (two per round, for independent work)
+      const uint32_t lend =
+          lbase + 64u * ((__reduce_max_sync(0xffffffffu, (oa - lbase) >> 6) + 1u) & ~1u);
+      for (uint32_t la = lbase; la < lend; la += 128u) {
+        float4 q[2];
 #pragma unroll
-      for (int kk = 0; kk < kChunk / 4; ++kk) test_quad(quads[kk]);
-    } else {
+        for (int j = 0; j < 2; ++j) {
+          const uint32_t e = la + 64u * j < oa ? lds_u16(la + 64u * j) : far;
+          q[j] = lds_f4(eb + 16u * e);
+        }
 #pragma unroll
-      for (int kk = 0; kk < kChunk / 4; ++kk) {
-        if ((uint32_t)kk >= nsteps) break;
-        test_quad(quads[kk]);
+        for (int j = 0; j < 2; ++j) {
+          const float2 dx = make_float2(pa.x - q[j].x, pb.x - q[j].x);
+          const float2 dy = make_float2(pa.y - q[j].y, pb.y - q[j].y);
+          const float2 dz = make_float2(pa.z - q[j].z, pb.z - q[j].z);
+          const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+          const int tj = NT == 1 ? 0 : __float_as_int(q[j].w);
+          if constexpr (kPacked) {
+            if (NT == 2) {
+              // both candidate types' parameters wait in registers
+              const bool k = tj != 0;
+              s2 = make_float2(k ? l1a.x : l0a.x, k ? l1b.x : l0b.x);
+              e24 = make_float2(k ? l1a.y : l0a.y, k ? l1b.y : l0b.y);
+              rca = __float_as_uint(k ? l1a.z : l0a.z);
+              rcb = __float_as_uint(k ? l1b.z : l0b.z);
+            } else if (NT > 2) {
+              const float4 la = d.lj4[ta + tj], lb = d.lj4[tbt + tj];
+              s2 = make_float2(la.x, lb.x);
+              e24 = make_float2(la.y, lb.y);
+              rca = __float_as_uint(la.z);
+              rcb = __float_as_uint(lb.z);
+            }
+            const bool ina = inside(r2.x, rca), inb = inside(r2.y, rcb);
+            float2 r2c = r2;
+            if (MODE == kModeCapped) {
+              const float2 fl = __fmul2_rn(make_float2(0.25f, 0.25f), s2);
+              r2c = make_float2(fmaxf(r2.x, fl.x), fmaxf(r2.y, fl.y));
+            }
+            const float2 inv = make_float2(rcp_approx(r2c.x), rcp_approx(r2c.y));
+            const float2 sr2 = __fmul2_rn(s2, inv);
+            const float2 sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
+            const float2 tt = __ffma2_rn(__fadd2_rn(e24, e24), sr6, make_float2(-e24.x, -e24.y));
+            float2 f = __fmul2_rn(__fmul2_rn(tt, sr6), inv);
+            f.x = ina ? f.x : 0.0f;
+            f.y = inb ? f.y : 0.0f;
+            if constexpr (kSum32) {
+              acc.fx = __ffma2_rn(f, dx, acc.fx);
+              acc.fy = __ffma2_rn(f, dy, acc.fy);
+              acc.fz = __ffma2_rn(f, dz, acc.fz);
+            } else {
+              const float2 gx = __fmul2_rn(f, dx), gy = __fmul2_rn(f, dy), gz = __fmul2_rn(f, dz);
+              acca.fx += (Acc)gx.x;
+              acca.fy += (Acc)gy.x;
+              acca.fz += (Acc)gz.x;
+              accb.fx += (Acc)gx.y;
+              accb.fy += (Acc)gy.y;
+              accb.fz += (Acc)gz.y;
+            }
+            if (ENERGY) {
+              const int ka = ta + tj, kb = tbt + tj;
+              const float2 e4 = make_float2(d.lj.e4[ka], d.lj.e4[kb]);
+              float2 u = __fmul2_rn(__fmul2_rn(e4, sr6), __fadd2_rn(sr6, m1));
+              u.x = ina ? u.x : 0.0f;
+              u.y = inb ? u.y : 0.0f;
+              const float2 us = make_float2(ina ? u.x - d.lj.ush[ka] : 0.0f,
+                                            inb ? u.y - d.lj.ush[kb] : 0.0f);
+              // f is zero outside the cutoff, where r^2 may be +inf
+              const float2 w = make_float2(ina ? f.x * r2c.x : 0.0f, inb ? f.y * r2c.y : 0.0f);
+              acca.pe += (Acc)(0.5f * u.x);
+              accb.pe += (Acc)(0.5f * u.y);
+              acca.pes += (Acc)(0.5f * us.x);
+              accb.pes += (Acc)(0.5f * us.y);
+              acca.vir += (Acc)(0.5f * w.x);
+              accb.vir += (Acc)(0.5f * w.y);
+              acca.n += (uint32_t)ina + (uint32_t)inb;
+            }
+          } else {
+            if (r2.x < d.lj.rc2[ta + tj] && r2.x > 0.0f)
+              acca.add(d.lj, ta + tj, dx.x, dy.x, dz.x, r2.x);
+            if (r2.y < d.lj.rc2[tbt + tj] && r2.y > 0.0f)
+              accb.add(d.lj, tbt + tj, dx.y, dy.y, dz.y, r2.y);
+          }
+        }
       }
-    }
+    } while (u < cb4);
   }
-  flush((oa - lbase) >> 6);
-  __syncwarp();
-  float fx, fy, fz;
-  Acc e0 = 0, e1 = 0, e2 = 0;
-  uint32_t e3 = 0;
-  if constexpr (kPacked) {
-    fx = acc2.fx.x + acc2.fx.y;
-    fy = acc2.fy.x + acc2.fy.y;
-    fz = acc2.fz.x + acc2.fz.y;
-#pragma unroll
-    for (int o = 8; o < 32; o <<= 1) {
-      fx += __shfl_xor_sync(0xffffffffu, fx, o);
-      fy += __shfl_xor_sync(0xffffffffu, fy, o);
-      fz += __shfl_xor_sync(0xffffffffu, fz, o);
-    }
-    if (ENERGY) {
-      e0 = acc2.pe.x + acc2.pe.y;
-      e1 = acc2.pes.x + acc2.pes.y;
-      e2 = acc2.vir.x + acc2.vir.y;
-      e3 = acc2.n;
-    }
-  } else {
-    // combine the 4 partial sums of each home atom (lanes il, il+8, il+16, il+24)
-#pragma unroll
-    for (int o = 8; o < 32; o <<= 1) {
-      acc.fx += __shfl_xor_sync(0xffffffffu, acc.fx, o);
-      acc.fy += __shfl_xor_sync(0xffffffffu, acc.fy, o);
-      acc.fz += __shfl_xor_sync(0xffffffffu, acc.fz, o);
-    }
-    fx = (float)acc.fx;
-    fy = (float)acc.fy;
-    fz = (float)acc.fz;
-    if (ENERGY) {
-      e0 = acc.pe;
-      e1 = acc.pes;
-      e2 = acc.vir;
-      e3 = acc.n;
-    }
+  // the 4 lanes of an atom
+  using Sum = typename std::conditional<kPacked && kSum32, float, Acc>::type;
+  Sum v[6] = {(Sum)acca.fx, (Sum)acca.fy, (Sum)acca.fz, (Sum)accb.fx, (Sum)accb.fy, (Sum)accb.fz};
+  if constexpr (kPacked && kSum32) {
+    v[0] = acc.fx.x;
+    v[1] = acc.fy.x;
+    v[2] = acc.fz.x;
+    v[3] = acc.fx.y;
+    v[4] = acc.fy.y;
+    v[5] = acc.fz.y;
   }
-  if (valid && q == 0) b.F[pi] = make_float4(fx, fy, fz, 0.0f);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    v[k] += __shfl_xor_sync(0xffffffffu, v[k], 1);
+    v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
+  }
+  if (t == 0 && va) b.F[pi] = make_float4((float)v[0], (float)v[1], (float)v[2], 0.0f);
+  if (t == 1 && vb) b.F[pi] = make_float4((float)v[3], (float)v[4], (float)v[5], 0.0f);
   if (ENERGY) {
-    ce[0] = warp_sum((double)e0);
-    ce[1] = warp_sum((double)e1);
-    ce[2] = warp_sum((double)e2);
-    ce[3] = (double)warp_sum(e3);
-  }
-}
-
-// One cluster, one atom type, FP32 sums, LJ or capped law.  Phase 1 tests
-// the quads as consume_cluster does but appends a quad, not a candidate: one
-// 4-byte entry per quad with at least one admitted candidate, in a per-lane
-// list laid out lane-minor (entry k of lane l at 128 k + 4 l, one bank per
-// lane).  Phase 2 evaluates the 4 candidates of every listed quad in packed
-// FP32x2 and keeps the ones inside the exact cutoff; a far atom of the quad
-// (a run's padding) has r^2 = +inf and is dropped by the same test.
-template <bool ENERGY, int MODE>
-__device__ __forceinline__ void consume_cluster_quads(const ForceBufs &b, const ItemDesc<1> &d,
-                                                      const Planes &pl, uint32_t cl,
-                                                      uint16_t *mylist, uint16_t *tb,
-                                                      double (&ce)[4]) {
-  constexpr uint32_t kEntries = kListLen / 2;  // 4-byte entries per lane
-  const int lane = threadIdx.x & 31;
-  const int il = lane & 7, q = lane >> 3;
-  const float *X = pl.X, *Y = pl.Y, *Z = pl.Z;
-  const uint32_t H = d.H, hb = d.hb;
-  const uint32_t h = cl * 8 + il;
-  const bool valid = h < H;
-  const uint32_t hs = hb + (valid ? h : H - 1);
-  const float xi = valid ? X[hs] : kNoAtom;
-  const float yi = valid ? Y[hs] : kNoAtom;
-  const float zi = valid ? Z[hs] : kNoAtom;
-  const uint32_t pi = valid && q == 0 ? __ldg(b.pid + d.home_g0 + h) : 0u;
-  const uint32_t Q = d.Q[cl], M = d.M[cl];
-  const uint32_t magic = 0xffffffffu / M + 1u;
-  for (uint32_t idx = lane; idx < 9u * M; idx += 32) {
-    const uint32_t c = __umulhi(idx, magic), i = idx - c * M;
-    if (i < d.len[cl][c]) tb[table_pos(d.pre[cl][c] + i)] = (uint16_t)(d.q0[cl][c] + i);
-  }
-  for (uint32_t u = Q + lane; u < ((Q + 15u) & ~15u); u += 32)
-    tb[table_pos(u)] = (uint16_t)d.sentinel;
-  __syncwarp();
-
-  const float rc2 = d.lj.rc2[0];
-  const float2 nrc = make_float2(-rc2 * (1.0f + 1.0f / 1024.0f), -rc2 * (1.0f + 1.0f / 1024.0f));
-  const float2 m1 = make_float2(-1.0f, -1.0f), two = make_float2(2.0f, 2.0f);
-  const float2 half = make_float2(0.5f, 0.5f);
-  const float2 s2 = make_float2(d.lj.s2[0], d.lj.s2[0]);
-  const float2 e24 = make_float2(d.lj.e24[0], d.lj.e24[0]);
-  const float2 e4 = make_float2(d.lj.e4[0], d.lj.e4[0]);
-  const float ush = d.lj.ush[0];
-  const float2 xi2 = make_float2(xi, xi), yi2 = make_float2(yi, yi), zi2 = make_float2(zi, zi);
-  const uint32_t xa = smem_u32(X), ya = smem_u32(Y), za = smem_u32(Z);
-  const uint32_t lbase = smem_u32(mylist) + 4u * (uint32_t)lane;
-  PairAcc2<ENERGY> a;
-  // two candidates of a listed quad: force (and energy) inside the exact cutoff
-  auto pair2 = [&](float2 dx, float2 dy, float2 dz) {
-    const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-    const bool ina = r2.x < rc2 && r2.x > 0.0f, inb = r2.y < rc2 && r2.y > 0.0f;
-    float2 r2c = r2;
-    if (MODE == kModeCapped) {
-      const float2 fl = __fmul2_rn(make_float2(0.25f, 0.25f), s2);
-      r2c = make_float2(fmaxf(r2.x, fl.x), fmaxf(r2.y, fl.y));
-    }
-    const float2 inv = make_float2(rcp_approx(r2c.x), rcp_approx(r2c.y));
-    const float2 sr2 = __fmul2_rn(s2, inv);
-    const float2 sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
-    const float2 t = __ffma2_rn(two, sr6, m1);
-    float2 f = __fmul2_rn(__fmul2_rn(__fmul2_rn(e24, sr6), t), inv);
-    f.x = ina ? f.x : 0.0f;
-    f.y = inb ? f.y : 0.0f;
-    a.fx = __ffma2_rn(f, dx, a.fx);
-    a.fy = __ffma2_rn(f, dy, a.fy);
-    a.fz = __ffma2_rn(f, dz, a.fz);
-    if (ENERGY) {
-      float2 u = __fmul2_rn(__fmul2_rn(e4, sr6), __fadd2_rn(sr6, m1));
-      u.x = ina ? u.x : 0.0f;
-      u.y = inb ? u.y : 0.0f;
-      float2 us = __fadd2_rn(u, make_float2(-ush, -ush));
-      us.x = ina ? us.x : 0.0f;
-      us.y = inb ? us.y : 0.0f;
-      a.pe = __ffma2_rn(half, u, a.pe);
-      a.pes = __ffma2_rn(half, us, a.pes);
-      // f is zero outside the cutoff, where r^2 may be +inf
-      float2 w = __fmul2_rn(__fmul2_rn(half, f), r2c);
-      w.x = ina ? w.x : 0.0f;
-      w.y = inb ? w.y : 0.0f;
-      a.vir = __fadd2_rn(a.vir, w);
-      a.n += (uint32_t)ina + (uint32_t)inb;
-    }
-  };
-  auto flush = [&](uint32_t cnt) {
-    const uint32_t steps = __reduce_max_sync(0xffffffffu, cnt);
-    for (uint32_t k = 0; k < steps; ++k) {
-      const uint32_t quad = k < cnt ? lds_u32(lbase + 128u * k) : d.sentinel;
-      const float4 x4 = lds_f4(xa + quad * 16u), y4 = lds_f4(ya + quad * 16u),
-                   z4 = lds_f4(za + quad * 16u);
-      pair2(__ffma2_rn(make_float2(x4.x, x4.y), m1, xi2),
-            __ffma2_rn(make_float2(y4.x, y4.y), m1, yi2),
-            __ffma2_rn(make_float2(z4.x, z4.y), m1, zi2));
-      pair2(__ffma2_rn(make_float2(x4.z, x4.w), m1, xi2),
-            __ffma2_rn(make_float2(y4.z, y4.w), m1, yi2),
-            __ffma2_rn(make_float2(z4.z, z4.w), m1, zi2));
-    }
-  };
-  uint32_t oa = lbase;  // shared-memory address of this lane's next entry
-  for (uint32_t u0 = 0; u0 < Q; u0 += kChunk) {
-    const uint32_t cnt = (oa - lbase) >> 7;
-    if (__reduce_max_sync(0xffffffffu, cnt) > kEntries - kChunk / 4) {
-      flush(cnt);
-      __syncwarp();
-      oa = lbase;
-    }
-    const uint2 qq = *reinterpret_cast<const uint2 *>(tb + u0 + 4 * q);
-    const uint32_t quads[4] = {qq.x & 0xffffu, qq.x >> 16, qq.y & 0xffffu, qq.y >> 16};
-    const uint32_t nsteps = min((Q - u0 + 3u) >> 2, (uint32_t)(kChunk / 4));
-    // one quad: 4 candidate tests; the quad is stored, and kept when any
-    // candidate is admitted (sign bit of r^2 - rc^2 (1 + 2^-10))
-    auto test_quad = [&](uint32_t quad) {
-      const float4 x4 = lds_f4(xa + quad * 16u), y4 = lds_f4(ya + quad * 16u),
-                   z4 = lds_f4(za + quad * 16u);
-      const float2 dxa = __ffma2_rn(make_float2(x4.x, x4.y), m1, xi2);
-      const float2 dxb = __ffma2_rn(make_float2(x4.z, x4.w), m1, xi2);
-      const float2 dya = __ffma2_rn(make_float2(y4.x, y4.y), m1, yi2);
-      const float2 dyb = __ffma2_rn(make_float2(y4.z, y4.w), m1, yi2);
-      const float2 dza = __ffma2_rn(make_float2(z4.x, z4.y), m1, zi2);
-      const float2 dzb = __ffma2_rn(make_float2(z4.z, z4.w), m1, zi2);
-      const float2 da = __ffma2_rn(dza, dza, __ffma2_rn(dya, dya, __ffma2_rn(dxa, dxa, nrc)));
-      const float2 db = __ffma2_rn(dzb, dzb, __ffma2_rn(dyb, dyb, __ffma2_rn(dxb, dxb, nrc)));
-      const uint32_t any = (__float_as_uint(da.x) | __float_as_uint(da.y) |
-                            __float_as_uint(db.x) | __float_as_uint(db.y)) >> 31;
-      sts_u32(oa, quad);
-      oa += any << 7;
-    };
-    if (nsteps == (uint32_t)(kChunk / 4)) {
-#pragma unroll
-      for (int kk = 0; kk < kChunk / 4; ++kk) test_quad(quads[kk]);
-    } else {
-#pragma unroll
-      for (int kk = 0; kk < kChunk / 4; ++kk) {
-        if ((uint32_t)kk >= nsteps) break;
-        test_quad(quads[kk]);
-      }
-    }
-  }
-  flush((oa - lbase) >> 7);
-  __syncwarp();
-  float fx = a.fx.x + a.fx.y, fy = a.fy.x + a.fy.y, fz = a.fz.x + a.fz.y;
-#pragma unroll
-  for (int o = 8; o < 32; o <<= 1) {
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
-  }
-  if (valid && q == 0) b.F[pi] = make_float4(fx, fy, fz, 0.0f);
-  if (ENERGY) {
-    ce[0] = warp_sum((double)(a.pe.x + a.pe.y));
-    ce[1] = warp_sum((double)(a.pes.x + a.pes.y));
-    ce[2] = warp_sum((double)(a.vir.x + a.vir.y));
-    ce[3] = (double)warp_sum(a.n);
+    const double e[4] = {warp_sum((double)(acca.pe + accb.pe)),
+                         warp_sum((double)(acca.pes + accb.pes)),
+                         warp_sum((double)(acca.vir + accb.vir)),
+                         (double)warp_sum(acca.n + accb.n)};
+    if (lane == 0)
+      for (int k = 0; k < 4; ++k) ce[k] = e[k];
   }
 }
 
 // Global-memory path of an item whose stage does not fit: task t covers the
 // groups of 32 consecutive home atoms t, t + ntask, ...; lanes are atoms.
 template <int NT, bool ENERGY, typename Acc, int MODE>
-__device__ void consume_task_global(const ForceBufs &b, const ItemDesc<NT> &d, uint32_t t,
-                                    double (&ce)[4]) {
+__device__ __noinline__ void task_global(const ForceBufs &b, const Stage<NT> &d, uint32_t t,
+                                         uint32_t ntask, double *ce) {
   const int lane = threadIdx.x & 31;
   const int nseg = d.nseg, z0 = d.z0, nz = d.nz;
-  const uint32_t hbeg = d.off[4][1];
   const uint32_t H = d.H;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (uint32_t gi = t; gi * 32 < H; gi += d.ntask) {
+  for (uint32_t gi = t; gi * 32 < H; gi += ntask) {
     const uint32_t h = gi * 32 + lane;
     const bool valid = h < H;
-    const uint32_t hh = valid ? h : H - 1;
+    const uint32_t gh = d.home_g0 + (valid ? h : H - 1);
     // home cell (staged index k in [1, nseg]) of this lane, and the warp's span
     int lo = 1, hi = nseg;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (d.off[4][mid] - hbeg <= hh) lo = mid; else hi = mid - 1;
+      if (b.start[d.kbase[4] + (uint32_t)(z0 - 1 + mid)] <= gh) lo = mid; else hi = mid - 1;
     }
     const int kmin = __reduce_min_sync(0xffffffffu, lo);
     const int kmax = __reduce_max_sync(0xffffffffu, lo);
-    const uint32_t gh = d.home_g0 + hh;
     const float4 p = b.rs[gh];
-    const float xi = p.x - d.sx[4], yi = p.y - d.sy[4], zi = p.z - d.sz_mid;
+    const float xi = p.x - d.sx[4], yi = p.y - d.sy[4], zi = p.z - d.szm;
     const int ti = NT == 1 ? 0 : __float_as_int(p.w);
     PairAcc<NT, ENERGY, Acc, MODE> acc;
     for (int c = 0; c < 9; ++c) {
       if (!d.periodic && d.kbase[c] == kNoCell) continue;  // no column past an open face
+      const float sx = d.sx[c], sy = d.sy[c];
       for (int k = kmin - 1; k <= kmax + 1; ++k) {
         const int zr = z0 - 1 + k, zc = (zr + nz) % nz;
         if (!d.periodic && (zr < 0 || zr >= nz)) continue;
         const uint32_t key = d.kbase[c] + (uint32_t)zc;
-        const float sz = k == 0 ? d.sz_lo : (k == nseg + 1 ? d.sz_hi : d.sz_mid);
+        const float sz = zr < 0 ? d.szl : (zr >= nz ? d.szh : d.szm);
         if (c == 4)
           global_range<NT, ENERGY, true, Acc, MODE>(b.rs, b.start[key], b.start[key + 1], xi, yi,
-                                                    zi, ti, d.sx[c], d.sy[c], sz, gh, d.lj, acc);
+                                                    zi, ti, sx, sy, sz, gh, d.lj, acc);
         else
           global_range<NT, ENERGY, false, Acc, MODE>(b.rs, b.start[key], b.start[key + 1], xi,
-                                                     yi, zi, ti, d.sx[c], d.sy[c], sz, 0, d.lj,
-                                                     acc);
+                                                     yi, zi, ti, sx, sy, sz, 0, d.lj, acc);
       }
     }
     if (valid) b.F[b.pid[gh]] = make_float4((float)acc.fx, (float)acc.fy, (float)acc.fz, 0.0f);
@@ -925,208 +744,105 @@ __device__ void consume_task_global(const ForceBufs &b, const ItemDesc<NT> &d, u
       s[3] += (double)warp_sum(valid ? acc.n : 0u);
     }
   }
-  for (int k = 0; k < 4; ++k) ce[k] = s[k];
+  if (ENERGY && lane == 0)
+    for (int k = 0; k < 4; ++k) ce[k] = s[k];
 }
 
 // ---- the kernel ---------------------------------------------------------------
 
-template <int NT, bool ENERGY, typename Acc, int kProd, int kCons, int MODE>
-__global__ void __launch_bounds__((kProd + kCons) * 32, (kProd + kCons) >= 16 ? 1 : 2)
-    k_force(ForceBufs b) {
+template <int NT, bool ENERGY, typename Acc, int kWarps, int MODE>
+__global__ void __launch_bounds__(kWarps * 32,
+                                  (NT == 1 && !ENERGY && std::is_same<Acc, float>::value && MODE != kModeSoftCore ? 32 : 24) / kWarps)
+    k_force(const __grid_constant__ ForceBufs b) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ ItemDesc<NT> desc[2];
-  __shared__ Scratch sc;
-  __shared__ uint64_t full[2], empty[2];
-  __shared__ double cle[2][kWinCap][4];
-  __shared__ int abort_flag, wait_ok;
-  __shared__ uint32_t next_item;
-
-  const uint32_t slots = padded_slots((uint32_t)b.cap);
-  const uint32_t pbytes = plane_bytes(slots, NT), wbytes = warp_bytes(slots);
-  // stage buffer k (computed, not indexed, so it stays in registers)
-  auto planes = [&](int k) {
-    float *base = reinterpret_cast<float *>(smem_raw + (size_t)k * pbytes);
-    Planes p;
-    p.X = base;
-    p.Y = base + slots;
-    p.Z = base + 2 * slots;
-    p.T = NT > 1 ? reinterpret_cast<uint32_t *>(base + 3 * slots) : nullptr;
-    return p;
-  };
+  __shared__ Stage<NT> d;
+  __shared__ uint64_t full;
+  __shared__ double cle[ENERGY ? kWinCap : 1][4];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t polls = b.wait_polls ? b.wait_polls : kWaitPolls;
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 2; ++k) {
-      mbar_init(&full[k], 1);
-      mbar_init(&empty[k], kCons);
-    }
-    abort_flag = 0;
-    mbar_fence_init();
-  }
-  __syncthreads();
-  const volatile int *abort_v = &abort_flag;
-
-  if (warp < kProd) {
-    // producers: wait for a free buffer (thread 0 polls; the group learns the
-    // outcome through its barrier), then stage the next item into it
-    auto wait_empty = [&](int bf, uint32_t parity) -> bool {
-      if (threadIdx.x == 0) {
-        const bool ok = mbar_wait_or_abort(&empty[bf], parity, &kNeverAbort, polls);
-        wait_ok = ok;
-        if (!ok) {
-          atomicOr(&b.status[desc[bf].sys], kStatusWaitTimeout);
-          abort_flag = 1;
-        }
-      }
-      producer_sync<kProd>();
-      const bool ok = wait_ok;
-      producer_sync<kProd>();
-      return ok;
-    };
-    // Items are claimed from a global counter (queue[0]), so that a CTA that
-    // runs faster than the other CTA on its SM takes more of them (the result
-    // of an item does not depend on which CTA computes it).  A CTA that will
-    // claim no more counts itself in queue[1]; the last one resets both for
-    // the next launch.
-    auto done_claiming = [&]() {
-      if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(b.queue + 1, 1u) == gridDim.x - 1) {
-          atomicExch(b.queue, 0u);
-          atomicExch(b.queue + 1, 0u);
-        }
-      }
-    };
-    uint32_t running = 0;
-    uint32_t n = 0;
-    for (;; ++n) {
-      if (threadIdx.x == 0) next_item = atomicAdd(b.queue, 1u);
-      const int bf = n & 1;
-      if (n >= 2) {
-        // the consumers are done with item n - 2 in this buffer
-        if (!wait_empty(bf, ((n >> 1) - 1) & 1u)) {
-          done_claiming();
-          return;
-        }
-        if (ENERGY && threadIdx.x == 0) write_partials(b, desc[bf], cle[bf]);
-      }
-      producer_sync<kProd>();
-      const uint32_t item = next_item;
-      producer_sync<kProd>();
-      if (item >= b.nitems) {
-        // no item left: an end marker in this buffer stops the consumers
-        done_claiming();
-        if (threadIdx.x == 0) {
-          desc[bf].item = kNone;
-          mbar_arrive(&full[bf]);
-        }
-        break;
-      }
-      const bool ok = produce_item<NT, MODE, kProd, kCons>(
-          b, item, desc[bf], sc, planes(bf), running);
-      if (!ok) {
-        done_claiming();
-        if (threadIdx.x == 0) abort_flag = 1;
-        return;
-      }
-      // test hook (failure-detection test entry only): withhold the first
-      // hand-off so that the consumers' bounded wait runs out
-      const bool withhold = (b.test_flags & 1u) && n == 0;
-      if (threadIdx.x == 0 && !withhold) mbar_arrive(&full[bf]);
-    }
-    // the last item: wait for the consumers, then its energy partials
-    if (n >= 1) {
-      const uint32_t m = n - 1;
-      const int bf = m & 1;
-      if (!wait_empty(bf, (m >> 1) & 1u)) return;
-      if (ENERGY && threadIdx.x == 0) write_partials(b, desc[bf], cle[bf]);
-    }
+  const ForceItem &it = b.items[blockIdx.x];
+  const uint32_t sys = it.sys;
+  if (b.steps_left != nullptr && b.steps_left[sys] == 0) {
+    // a system whose step budget is spent keeps its state
+    if (ENERGY && threadIdx.x < 4) b.partials[(size_t)blockIdx.x * 4 + threadIdx.x] = 0.0;
     return;
   }
-
-  // consumers
-  const int cw = warp - kProd;
-  uint16_t *mylist =
-      reinterpret_cast<uint16_t *>(smem_raw + 2 * (size_t)pbytes + (size_t)cw * wbytes);
-  uint16_t *tb = mylist + 32 * kListLen;
-  for (uint32_t n = 0;; ++n) {
-    const int bf = n & 1;
-    bool ok = lane != 0 || mbar_wait_or_abort(&full[bf], (n >> 1) & 1u, abort_v, polls);
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    if (!ok) {
-      if (lane == 0 && !*abort_v) atomicOr(&b.status[0], kStatusWaitTimeout);
-      return;
-    }
-    const ItemDesc<NT> &d = desc[bf];
-    if (d.item == kNone) break;  // end marker
-    const Planes pbuf = planes(bf);
-    if (!d.skip) {
-      if (!d.overflow) {
-        // clusters go round-robin over the CTA's whole item sequence
-        const uint32_t first = ((uint32_t)cw + (uint32_t)kCons - d.base) % (uint32_t)kCons;
-        for (uint32_t cl = first; cl < d.nclus; cl += kCons) {
-          double ce[4];
-          if constexpr (NT == 1 && std::is_same<Acc, float>::value && MODE != kModeSoftCore)
-            consume_cluster_quads<ENERGY, MODE>(b, d, pbuf, cl, mylist, tb, ce);
-          else
-            consume_cluster<NT, ENERGY, Acc, MODE>(b, d, pbuf, cl, mylist, tb, ce);
-          if (ENERGY && lane == 0)
-            for (int k = 0; k < 4; ++k) cle[bf][cl][k] = ce[k];
-        }
-      } else {
-        for (uint32_t t = (uint32_t)cw; t < d.ntask; t += kCons) {
-          double ce[4];
-          consume_task_global<NT, ENERGY, Acc, MODE>(b, d, t, ce);
-          if (ENERGY && lane == 0)
-            for (int k = 0; k < 4; ++k) cle[bf][t][k] = ce[k];
-        }
-      }
+  const uint32_t slots = padded_slots((uint32_t)b.cap);
+  float4 *E = reinterpret_cast<float4 *>(smem_raw);
+  uint2 *Hf = reinterpret_cast<uint2 *>(smem_raw + (size_t)slots * 16u);
+  uint32_t *Ht = reinterpret_cast<uint32_t *>(smem_raw + (size_t)slots * 24u);
+  float *zb = reinterpret_cast<float *>(smem_raw + (size_t)slots * (slot_bytes(NT) - 1u));
+  uint32_t *tab = reinterpret_cast<uint32_t *>(smem_raw + (size_t)slots * slot_bytes(NT)) +
+                  warp * (warp_bytes(NT) / 4);
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_init(&full, 1);
+      mbar_fence_init();
     }
     __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[bf]);
+    plan_stage<NT>(b, it, d, E, &full);
+  } else if (warp == 1) {
+    plan_frame<NT>(b, it, d);
+  } else if (warp == 2) {
+    load_lj<NT, MODE>(b, b.sys[sys], d);
+  }
+  __syncthreads();
+  if (!d.overflow) {
+    bool ok = lane != 0 || mbar_wait_or_abort(&full, 0u, &kNeverAbort,
+                                              b.wait_polls ? b.wait_polls : kWaitPolls);
+    ok = __syncthreads_and(ok);
+    if (!ok) {
+      // the copies did not arrive: report it, and give them one more bounded
+      // wait before the shared memory they write is released
+      if (threadIdx.x == 0) {
+        atomicOr(&b.status[sys], kStatusWaitTimeout);
+        if (!(b.test_flags & 1u)) mbar_wait_bounded(&full, 0u);
+      }
+      return;
+    }
+    if (d.shifted) {
+      shift_stage<NT, kWarps>(d, E);
+      __syncthreads();
+    }
+    make_records<NT, kWarps>(d, E, Hf, Ht, zb);
+    __syncthreads();
+  }
+  // records out of the fp16 range (atoms far outside their cells): global path
+  const bool global = d.overflow || __uint_as_float(d.nmax) > kMaxNorm;
+  const uint32_t ntile = d.ntile;
+  for (uint32_t k = warp; k < ntile; k += kWarps) {
+    double *ce = cle[ENERGY ? k : 0];
+    if (!global)
+      tile_forces<NT, ENERGY, Acc, MODE>(b, d, E, Hf, Ht, zb, k, tab, ce);
+    else
+      task_global<NT, ENERGY, Acc, MODE>(b, d, k, ntile, ce);
+  }
+  if (ENERGY) {  // the item's sums in tile order
+    __syncthreads();
+    if (threadIdx.x < 4) {
+      double v = 0.0;
+      for (uint32_t k = 0; k < ntile; ++k) v += cle[k][threadIdx.x];
+      b.partials[(size_t)blockIdx.x * 4 + threadIdx.x] = v;
+    }
   }
 }
 
-// CTAs per SM of a launch shape, from the occupancy calculator.
-template <typename K>
-int resident_ctas(K kern, int threads, size_t smem) {
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, threads, smem) != cudaSuccess) n = 1;
-  return n > 0 ? n : 1;
-}
+// Warps of a CTA: the default, and a small one.
+constexpr int kWarpsDefault = 8, kWarpsSmall = 4;
 
-int sm_count() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 1;
-  }
-  return n;
-}
-
-template <int NT, bool E, typename Acc, int P, int C, int MODE = kModeLJ>
+template <int NT, bool E, typename Acc, int kWarps, int MODE = kModeLJ>
 cudaError_t launch_w(const ForceBufs &b, cudaStream_t s) {
-  const size_t smem = smem_bytes((uint32_t)b.cap, C, NT);
-  auto kern = k_force<NT, E, Acc, P, C, MODE>;
+  const size_t smem = smem_bytes((uint32_t)b.cap, kWarps, NT);
+  auto kern = k_force<NT, E, Acc, kWarps, MODE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  // persistent grid: every resident CTA slot, at most one CTA per item
-  const long slots = (long)resident_ctas(kern, (P + C) * 32, smem) * sm_count();
-  const unsigned grid = (unsigned)std::min<long>(slots, (long)b.nitems);
-  return launch_pdl(kern, dim3(grid), dim3((P + C) * 32), smem, s, b);
+  return launch_pdl(kern, dim3(b.nitems), dim3(kWarps * 32), smem, s, b);
 }
-
-// Launch shapes (producer warps, consumer warps): the default, and a small one.
-constexpr int kProdDefault = 4, kConsDefault = 8;
-constexpr int kProdSmall = 2, kConsSmall = 4;
 
 template <int NT, bool E, typename Acc>
 cudaError_t launch_t(const ForceBufs &b, int threads, cudaStream_t s) {
-  return threads == 128 ? launch_w<NT, E, Acc, kProdSmall, kConsSmall>(b, s)
-                        : launch_w<NT, E, Acc, kProdDefault, kConsDefault>(b, s);
+  return threads == 128 ? launch_w<NT, E, Acc, kWarpsSmall>(b, s)
+                        : launch_w<NT, E, Acc, kWarpsDefault>(b, s);
 }
 
 template <int NT>
@@ -1143,10 +859,10 @@ template <int MODE>
 cudaError_t launch_mode(const ForceBufs &b, int nt_max, cudaStream_t s) {
   if (b.nitems == 0) return cudaSuccess;
   switch (nt_max) {
-    case 1: return launch_w<1, false, float, kProdDefault, kConsDefault, MODE>(b, s);
-    case 2: return launch_w<2, false, float, kProdDefault, kConsDefault, MODE>(b, s);
-    case 3: case 4: return launch_w<4, false, float, kProdDefault, kConsDefault, MODE>(b, s);
-    default: return launch_w<8, false, float, kProdDefault, kConsDefault, MODE>(b, s);
+    case 1: return launch_w<1, false, float, kWarpsDefault, MODE>(b, s);
+    case 2: return launch_w<2, false, float, kWarpsDefault, MODE>(b, s);
+    case 3: case 4: return launch_w<4, false, float, kWarpsDefault, MODE>(b, s);
+    default: return launch_w<8, false, float, kWarpsDefault, MODE>(b, s);
   }
 }
 
@@ -1154,33 +870,24 @@ cudaError_t launch_mode(const ForceBufs &b, int nt_max, cudaStream_t s) {
 
 int force_max_segment() { return kMaxSeg; }
 
-int force_max_capacity(int warps, int nt) {
+int force_max_capacity() {
   // largest staged-atom capacity whose shared memory fits one CTA
-  const int consumers = warps >= 8 ? kConsDefault : kConsSmall;
-  (void)kProdSmall;
   uint32_t cap = 64;
-  while (smem_bytes(cap + 64, consumers, nt) <= 180u * 1024u) cap += 64;
+  while (smem_bytes(cap + 64, kWarpsDefault, kMaxTypes) <= 180u * 1024u) cap += 64;
   return (int)cap;
 }
 
-// Static shared memory of a force CTA for up to `nt` types: the two item
-// descriptors, the producer scratch, the per-cluster energy sums, and 1 KB
-// for barriers and flags.
-template <int NT>
-constexpr uint32_t static_smem() {
-  return 2u * (uint32_t)sizeof(ItemDesc<NT>) + (uint32_t)sizeof(Scratch) +
-         2u * kWinCap * 4u * 8u + 1024u;
-}
-
 int force_smem_per_cta(int cap, int nt) {
-  const uint32_t st = nt <= 1 ? static_smem<1>() : nt <= 2 ? static_smem<2>()
-                      : nt <= 4 ? static_smem<4>() : static_smem<8>();
-  return (int)(smem_bytes((uint32_t)cap, kConsDefault, nt) + st);
+  // dynamic part, and a bound of the static part (stage record, energy sums)
+  const size_t st = nt <= 1 ? sizeof(Stage<1>) : nt <= 2 ? sizeof(Stage<2>)
+                    : nt <= 4 ? sizeof(Stage<4>) : sizeof(Stage<8>);
+  return (int)(smem_bytes((uint32_t)cap, kWarpsDefault, nt) + st + kWinCap * 4 * 8 + 64);
 }
 
-int force_smem_limit() {
-  // two CTAs per SM share its 228 KB, less 1 KB per CTA reserved by the driver
-  return 112 * 1024;
+int force_smem_limit(int nt) {
+  // the CTAs per SM that the registers allow (one type 4, several 3) share its
+  // 228 KB, less 1 KB per CTA reserved by the driver
+  return (nt <= 1 ? 56 : 74) * 1024;
 }
 
 int force_threads() { return 256; }

@@ -83,19 +83,21 @@ static const char *env_once(int slot) {
 }
 
 int choose_segment(double atoms_per_cell, int nz, double scale, int nt, bool half) {
-  // about 200 home atoms (25 clusters of 8) per force work item; PB_FORCE_SEG
-  // overrides.  Shorter runs while the stage would not let two force CTAs
-  // share an SM.
+  // full-shell kernel: 8 tiles of 16 home atoms, one per warp of a CTA, with
+  // room for a few atoms above the mean; half-shell kernel: about 200 home
+  // atoms.  PB_FORCE_SEG overrides.  Shorter runs while the stage would not
+  // leave the CTAs per SM that the kernel's launch shape is built for.
   const double apc = std::max(atoms_per_cell, 1.0);
-  int seg = (int)std::lround(200.0 * scale / apc);
+  int seg = half ? (int)std::lround(200.0 * scale / apc) : (int)std::lround(124.0 * scale / apc);
   if (const char *e = env_once(0)) seg = std::atoi(e);
   seg = std::max(1, std::min(seg, force_max_segment()));
   seg = std::min(seg, nz);
-  // the kernel that runs sets the limit; the full-shell one also serves the
-  // soft-core and relaxation forces, so it always has to fit
-  while (seg > 1 && (force_smem_per_cta(choose_capacity(apc, seg), nt) > force_smem_limit() ||
-                     (half && force_half_smem_per_cta(choose_capacity_half(apc, seg), nt) >
-                                  112 * 1024)))
+  // with the half shell, the full-shell kernel still serves the soft-core and
+  // relaxation forces, so it has to fit as well
+  while (seg > 1 &&
+         (force_smem_per_cta(choose_capacity(apc, seg), nt) >
+              (half ? 112 * 1024 : force_smem_limit(nt)) ||
+          (half && force_half_smem_per_cta(choose_capacity_half(apc, seg), nt) > 112 * 1024)))
     --seg;
   return seg;
 }
@@ -114,11 +116,11 @@ int choose_tile_atoms(double atoms_per_cell) {
 
 int choose_capacity(double atoms_per_cell, int seg) {
   const double expect = 9.0 * (seg + 2) * std::max(atoms_per_cell, 1.0);
-  double factor = 1.15;  // headroom over the mean occupancy; PB_FORCE_CAP overrides
+  double factor = 1.12;  // headroom over the mean occupancy; PB_FORCE_CAP overrides
   if (const char *e = env_once(1)) factor = std::atof(e);
-  const double cap = factor * expect + 128.0;
-  // the largest launch shape (8 warps, 8 types) bounds every launch's memory
-  static const double max_atoms = (double)force_max_capacity(8, kMaxTypes);
+  const double cap = factor * expect + 96.0;
+  // what one CTA can hold bounds every launch's memory
+  static const double max_atoms = (double)force_max_capacity();
   return (int)std::min(cap, max_atoms);
 }
 

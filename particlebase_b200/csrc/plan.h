@@ -26,10 +26,11 @@ void morton_columns(int nx, int ny, std::vector<uint32_t> &rank, std::vector<uin
 // neighbour outside the grid is kNoCell.
 void neighbor_table(const Grid &g, std::vector<uint32_t> &out);
 
-// z cells per force work item for a mean cell occupancy: about 200 * scale
-// home atoms per item, at most force_max_segment(), and short enough for two
-// force CTAs per SM with `nt` atom types.
-// `half`: the half-shell force kernel runs (its stage has to fit as well).
+// z cells per force work item for a mean cell occupancy: about 119 * scale
+// home atoms per item (8 tiles of 16), at most force_max_segment(), and short
+// enough for four force CTAs per SM with `nt` atom types.
+// `half`: the half-shell force kernel runs (about 200 * scale home atoms; its
+// stage has to fit as well).
 int choose_segment(double atoms_per_cell, int nz, double scale = 1.0, int nt = 1,
                    bool half = false);
 
@@ -52,14 +53,14 @@ void append_items(uint32_t sys, const Grid &g, int seg, uint32_t cell0,
                   std::vector<ForceItem> &items);
 
 int force_max_segment();
-// Largest staged-atom capacity of a force CTA of `warps` warps for `nt` types.
-int force_max_capacity(int warps, int nt);
+// Largest staged-atom capacity of a force CTA.
+int force_max_capacity();
 // Shared memory (dynamic plus an upper bound of the static part) of one
 // default-shape force CTA with staged-atom capacity `cap` and `nt` types.
 int force_smem_per_cta(int cap, int nt);
 // The shared memory a default-shape force CTA may use so that the CTAs per SM
 // its launch shape is built for stay resident.
-int force_smem_limit();
+int force_smem_limit(int nt);
 // The same two for the half-shell force kernel (force_half.cu).
 int force_half_max_capacity(int nt);
 int force_half_smem_per_cta(int cap, int nt);

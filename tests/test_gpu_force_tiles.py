@@ -100,3 +100,24 @@ def test_open_box_and_atoms_far_outside(cuda_lib, far):
         keep = ((d ** 2).sum(1) > 0.9) | (np.arange(s.n) == 90)  # no overlap with the moved atom
         s.r, s.v, s.mass, s.types = s.r[keep], s.v[keep], s.mass[keep], s.types[keep]
     assert check(s, periodic=False) == 0
+
+
+def test_non_finite_atoms_leave_the_others_alone(cuda_lib):
+    """NaN and infinite coordinates: no force on or from those atoms."""
+    from particlebase_b200.md import from_system
+    s = system((9.0, 10.5, 16.0), 800, 1, 9)
+    bad = {5: (np.nan, 1.0, 2.0), 77: (3.0, 3.0, np.nan), 200: (np.inf, 2.0, 2.0),
+           333: (1.0, -np.inf, 9.0), 640: (4.0, 5.0, np.inf), 641: (np.nan,) * 3}
+    p = from_system(s)
+    r = p.get("r")
+    for k, x in bad.items():
+        r[k, :3] = x
+    p.set("r", r)
+    p.calcBlockID()
+    p.calcForce()
+    got = p.get("F")[:, :3].astype(np.float64)
+    keep = np.setdiff1d(np.arange(s.n), list(bad))
+    assert (got[list(bad)] == 0).all()
+    s.r, s.types = s.r[keep], s.types[keep]
+    F, _ = all_pairs(s)
+    assert np.sqrt(((got[keep] - F) ** 2).sum()) < BAR * np.sqrt((F ** 2).sum())
