@@ -225,7 +225,7 @@ __device__ __forceinline__ void canon_cell(const CellBufs &b, const uint32_t *me
   if (li < (int)n) {
     const uint32_t s = s0 + rank;
     b.pid[s] = me;
-    b.slot[me] = s;
+    if (b.slot) b.slot[me] = s;
     b.rs[s] = make_float4(p.x, p.y, p.z, __int_as_float((int)b.type[me]));
     if (b.xs) write_mirror(b, me, s, p, key);
   }
@@ -245,7 +245,7 @@ __device__ void canon_large(const CellBufs &b, const uint32_t *mem, uint32_t s0,
     }
     const uint32_t s = s0 + rank;
     b.pid[s] = me;
-    b.slot[me] = s;
+    if (b.slot) b.slot[me] = s;
     b.rs[s] = make_float4(p.x, p.y, p.z, __int_as_float((int)b.type[me]));
     if (b.xs) write_mirror(b, me, s, p, key);
   }
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
         for (uint32_t q = lo; q < hi; ++q) rank += canon_before(szk[q], sid[q], kz, me) ? 1u : 0u;
         const uint32_t s = base + lo + rank;
         b.pid[s] = me;
-        b.slot[me] = s;
+        if (b.slot) b.slot[me] = s;
         b.rs[s] = make_float4(p[u].x, p[u].y, p[u].z, __int_as_float((int)ty[u]));
         if (b.xs) write_mirror_of(b, b.sys[sy[u]], s, p[u], c0 + k, ty[u]);
       }

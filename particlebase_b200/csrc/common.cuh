@@ -52,6 +52,9 @@ struct LJTable {
 // predecessor has finished and its memory is visible (the same ordering as a
 // plain launch), then lets its own successor be scheduled.
 #ifdef __CUDACC__
+// A kernel may read ahead of that wait what neither its predecessor nor anything
+// the predecessor still waits for can write: its own launch began after the
+// predecessor's wait, so all earlier kernels have finished.
 __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

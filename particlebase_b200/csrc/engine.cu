@@ -246,7 +246,6 @@ void free_cells(Engine &e) {
   dfree(e, e.cctl);
   dfree(e, e.pid_tmp);
   dfree(e, e.pid);
-  dfree(e, e.slot);
   dfree(e, e.rs);
   dfree(e, e.xs);
   dfree(e, e.ys);
@@ -734,15 +733,19 @@ int engine_setup_cells(Engine &e) {
             dalloc(e, &e.cctl, 2) == cudaSuccess && dalloc(e, &e.pid_tmp, N) == cudaSuccess &&
             dalloc(e, &e.within, N) == cudaSuccess &&
             dalloc(e, &e.tilesum, (C + 4095) / 4096) == cudaSuccess &&
-            dalloc(e, &e.pid, N) == cudaSuccess && dalloc(e, &e.slot, N) == cudaSuccess &&
-            dalloc(e, &e.rs, N) == cudaSuccess && dalloc(e, &e.xs, e.mirrorN) == cudaSuccess &&
-            dalloc(e, &e.ys, e.mirrorN) == cudaSuccess && dalloc(e, &e.zs, e.mirrorN) == cudaSuccess &&
-            dalloc(e, &e.ts, e.mirrorN) == cudaSuccess && dalloc(e, &e.colrank, ncols) == cudaSuccess &&
+            dalloc(e, &e.pid, N) == cudaSuccess &&
+            dalloc(e, &e.rs, N) == cudaSuccess && dalloc(e, &e.colrank, ncols) == cudaSuccess &&
             dalloc(e, &e.colxy, ncols) == cudaSuccess &&
             dalloc(e, &e.d_sys, e.nsys) == cudaSuccess && dalloc(e, &e.d_items, nitems) == cudaSuccess &&
             dalloc(e, &e.d_item0, e.nsys + 1) == cudaSuccess &&
             dalloc(e, &e.fpartials, (size_t)4 * nitems) == cudaSuccess &&
             dalloc(e, &e.fqueue, 2) == cudaSuccess;
+  // the half-shell kernel stages from structure-of-arrays mirrors; nobody else
+  // reads them, so the cell build writes them only where that kernel runs
+  if (e.facc)
+    ok = ok && dalloc(e, &e.xs, e.mirrorN) == cudaSuccess &&
+         dalloc(e, &e.ys, e.mirrorN) == cudaSuccess &&
+         dalloc(e, &e.zs, e.mirrorN) == cudaSuccess && dalloc(e, &e.ts, e.mirrorN) == cudaSuccess;
   if (!ok) {
     free_cells(e);
     return fail(e, PB_ERR_OOM, "cell list allocation failed");
@@ -825,7 +828,6 @@ CellBufs engine_cbufs(Engine &e) {
   b.tile_atoms = e.tile_atoms;
   b.ctl = e.cctl;
   b.pid = e.pid;
-  b.slot = e.slot;
   b.rs = e.rs;
   b.xs = e.xs;
   b.ys = e.ys;

@@ -67,7 +67,7 @@ struct Engine {
   uint32_t ncells = 0;
   uint32_t *key = nullptr, *within = nullptr, *tilesum = nullptr, *count = nullptr,
            *start = nullptr, *pid_tmp = nullptr,
-           *pid = nullptr, *slot = nullptr, *colrank = nullptr, *colxy = nullptr,
+           *pid = nullptr, *colrank = nullptr, *colxy = nullptr,
            *d_item0 = nullptr;
   // cell buckets of the two-kernel build: bucket_cap ids per cell, the
   // overflow list, tile counts, and two control words

@@ -108,44 +108,77 @@ __device__ __forceinline__ void load_v(const IntegrateArgs &a, const SysInt &S, 
   }
 }
 
-// acc + m |v|^2 with every rounding written out: the steps and k_mv2 add the
-// same terms, so a temperature read after a step gives the same bits whichever
+// m |v|^2 with every rounding written out: the steps and k_mv2 add the same
+// terms, so a temperature read after a step gives the same bits whichever
 // kernel summed it (left to the compiler, their contractions differed).
-__device__ __forceinline__ double add_mv2(double acc, float m, double x, double y, double z) {
-  return __fma_rn((double)m, __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))), acc);
+__device__ __forceinline__ double mv2_term(float m, double x, double y, double z) {
+  return __dmul_rn((double)m, __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))));
 }
 
-__global__ void __launch_bounds__(kIntThreads) k_vv(IntegrateArgs a) {
+// The sums of one block from its atoms' terms.  An atom's terms are added, in
+// atom order, to the sum of thread t % kIntThreads; the wide form (a thread per
+// atom) hands them over in shared memory, so both forms give the same bits.
+template <int NV, int kT>
+struct Terms {
+  double s[NV];
+  __device__ __forceinline__ Terms() {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) s[k] = 0.0;
+  }
+  __device__ __forceinline__ void add(int k, double e) { s[k] = __dadd_rn(s[k], e); }
+  __device__ __forceinline__ void gather() {
+    if constexpr (kT != kIntThreads) {
+      __shared__ double sh[NV][kIntAtoms];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sh[k][threadIdx.x] = s[k];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        double v = 0.0;
+        if (threadIdx.x < kIntThreads)
+          for (int j = 0; j < kIntAtoms; j += kIntThreads) v = __dadd_rn(v, sh[k][j + threadIdx.x]);
+        s[k] = v;
+      }
+    }
+  }
+};
+
+// kT threads a block: kIntThreads (4 atoms each) or kIntAtoms (the wide form).
+// All arithmetic with its roundings written out, so that the forms agree.
+template <int kT>
+__global__ void __launch_bounds__(kT) k_vv(IntegrateArgs a) {
   pdl_enter();
   __shared__ double red[32];
   const BlockMap m = a.map[blockIdx.x];
   if (finished(a, m.sys)) return;
   const SysInt &S = a.sys[m.sys];
-  double mv2 = 0;
-  for (uint32_t t = threadIdx.x; t < m.n; t += kIntThreads) {
+  Terms<1, kT> sum;
+  for (uint32_t t = threadIdx.x; t < m.n; t += kT) {
     const uint32_t i = m.i0 + t;
     const float dt = S.dt;
     const float dt2 = dt * 0.5f;
-    const float h = dt2 * a.minv[i];  // dt / 2m
+    const float h = __fmul_rn(dt2, a.minv[i]);  // dt / 2m
     const float4 F = a.F[i], Fo = a.Fold[i];
     float4 v = a.v[i];
-    v.x += (F.x + Fo.x) * h;
-    v.y += (F.y + Fo.y) * h;
-    v.z += (F.z + Fo.z) * h;
+    v.x = fmaf(__fadd_rn(F.x, Fo.x), h, v.x);
+    v.y = fmaf(__fadd_rn(F.y, Fo.y), h, v.y);
+    v.z = fmaf(__fadd_rn(F.z, Fo.z), h, v.z);
     v.w = 0.f;
-    const float h2 = h * dt;
+    const float h2 = __fmul_rn(h, dt);
     float4 p = a.r[i];
-    p.x += v.x * dt + F.x * h2;
-    p.y += v.y * dt + F.y * h2;
-    p.z += v.z * dt + F.z * h2;
+    p.x = __fadd_rn(p.x, fmaf(v.x, dt, __fmul_rn(F.x, h2)));
+    p.y = __fadd_rn(p.y, fmaf(v.y, dt, __fmul_rn(F.y, h2)));
+    p.z = __fadd_rn(p.z, fmaf(v.z, dt, __fmul_rn(F.z, h2)));
     if (a.wrap) wrap3(S, p);
     a.v[i] = v;
     a.r[i] = p;
-    mv2 = add_mv2(mv2, a.mass[i], v.x, v.y, v.z);
+    sum.add(0, mv2_term(a.mass[i], v.x, v.y, v.z));
   }
-  double s[1] = {mv2}, tot[1];
-  block_sum<1>(s, red);
-  if (sys_total<1>(s, a.partials, blockIdx.x, S.blk0, S.nblk, &a.sc[m.sys].counter[0], tot, red)) {
+  sum.gather();
+  double tot[1];
+  block_sum<1>(sum.s, red);
+  if (sys_total<1>(sum.s, a.partials, blockIdx.x, S.blk0, S.nblk, &a.sc[m.sys].counter[0], tot,
+                   red)) {
     a.sc[m.sys].mv2 = tot[0];
     if (!isfinite(tot[0])) atomicOr(&a.status[m.sys], kStatusNonFinite);
     count_step(a, m.sys);  // every block of the system has read steps_left
@@ -153,13 +186,8 @@ __global__ void __launch_bounds__(kIntThreads) k_vv(IntegrateArgs a) {
 }
 
 // Per-atom inputs of the Gaussian passes, read through the read-only data
-// path.  A thread's atoms (kIntAtoms / kIntThreads, strided) are taken
-// kIntGroup at a time, the loads of a group issued before its arithmetic;
-// one atom at a time keeps the register count, and so the number of resident
-// threads, highest, which measured fastest.
-constexpr int kIntPer = kIntAtoms / kIntThreads;
-constexpr int kIntGroup = 1;
-
+// path.  A thread takes its atoms one at a time: that keeps the register count,
+// and so the number of resident threads, highest, which measured fastest.
 struct GaussIn {
   float4 F, Fo;
   double v[3];
@@ -179,17 +207,18 @@ __device__ __forceinline__ void gauss_load(const IntegrateArgs &a, const SysInt 
 // A = v + (F + Fold) dt/2m - v xi(t-dt) dt/2.
 __device__ __forceinline__ void gauss_A(const SysInt &S, const GaussIn &g, double hx,
                                         double A[3]) {
-  const float h = (S.dt * 0.5f) * g.minv;
-  A[0] = g.v[0] + (double)(g.F.x + g.Fo.x) * h - g.v[0] * hx;
-  A[1] = g.v[1] + (double)(g.F.y + g.Fo.y) * h - g.v[1] * hx;
-  A[2] = g.v[2] + (double)(g.F.z + g.Fo.z) * h - g.v[2] * hx;
+  const double h = __fmul_rn(S.dt * 0.5f, g.minv);
+  A[0] = __fma_rn(-g.v[0], hx, __fma_rn((double)__fadd_rn(g.F.x, g.Fo.x), h, g.v[0]));
+  A[1] = __fma_rn(-g.v[1], hx, __fma_rn((double)__fadd_rn(g.F.y, g.Fo.y), h, g.v[1]));
+  A[2] = __fma_rn(-g.v[2], hx, __fma_rn((double)__fadd_rn(g.F.z, g.Fo.z), h, g.v[2]));
 }
 
 // Eight blocks per SM: the first pass fits in 32 registers without spills, and
 // the extra resident warps keep more loads in flight (0.040 against 0.043 ms
 // for both passes at 1M atoms).  The second pass measured slower when held to
 // 40 or 32 registers, which spill.
-__global__ void __launch_bounds__(kIntThreads, 8) k_gauss_a(IntegrateArgs a) {
+template <int kT>
+__global__ void __launch_bounds__(kT, kT == kIntThreads ? 8 : 1) k_gauss_a(IntegrateArgs a) {
   pdl_enter();
   __shared__ double red[2 * 32];
   const BlockMap m = a.map[blockIdx.x];
@@ -198,29 +227,24 @@ __global__ void __launch_bounds__(kIntThreads, 8) k_gauss_a(IntegrateArgs a) {
   DevScalars &sc = a.sc[m.sys];
   const double xi_old = sc.xi_old;
   const double hx = (double)S.dt * 0.5 * xi_old;
-  double s[2] = {0, 0};
+  Terms<2, kT> sum;
 #pragma unroll
-  for (int j0 = 0; j0 < kIntPer; j0 += kIntGroup) {
-    GaussIn g[kIntGroup];
-#pragma unroll
-    for (int j = 0; j < kIntGroup; ++j) {
-      const uint32_t t = threadIdx.x + (j0 + j) * kIntThreads;
-      if (t < m.n) gauss_load(a, S, m.i0 + t, g[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < kIntGroup; ++j) {
-      const uint32_t t = threadIdx.x + (j0 + j) * kIntThreads;
-      if (t < m.n) {
-        double A[3];
-        gauss_A(S, g[j], hx, A);
-        s[0] += (double)g[j].F.x * A[0] + (double)g[j].F.y * A[1] + (double)g[j].F.z * A[2];
-        s[1] += (double)g[j].mass * (A[0] * A[0] + A[1] * A[1] + A[2] * A[2]);
-      }
+  for (int j = 0; j < kIntAtoms / kT; ++j) {
+    const uint32_t t = threadIdx.x + j * kT;
+    if (t < m.n) {
+      GaussIn g;
+      gauss_load(a, S, m.i0 + t, g);
+      double A[3];
+      gauss_A(S, g, hx, A);
+      sum.add(0, __fma_rn((double)g.F.z, A[2],
+                          __fma_rn((double)g.F.y, A[1], __dmul_rn((double)g.F.x, A[0]))));
+      sum.add(1, mv2_term(g.mass, A[0], A[1], A[2]));
     }
   }
+  sum.gather();
   double tot[2];
-  block_sum<2>(s, red);
-  if (sys_total<2>(s, a.partials, blockIdx.x, S.blk0, S.nblk, &sc.counter[1], tot, red)) {
+  block_sum<2>(sum.s, red);
+  if (sys_total<2>(sum.s, a.partials, blockIdx.x, S.blk0, S.nblk, &sc.counter[1], tot, red)) {
     const double hdt = 0.5 * (double)S.dt;
     const double c = tot[1] > 0 ? tot[0] / tot[1] : 0.0;
     double xi = (xi_old == 0.0) ? c : c / (1.0 - c * hdt);
@@ -234,7 +258,8 @@ __global__ void __launch_bounds__(kIntThreads, 8) k_gauss_a(IntegrateArgs a) {
   }
 }
 
-__global__ void __launch_bounds__(kIntThreads) k_gauss_b(IntegrateArgs a) {
+template <int kT>
+__global__ void __launch_bounds__(kT) k_gauss_b(IntegrateArgs a) {
   pdl_enter();
   __shared__ double red[32];
   const BlockMap m = a.map[blockIdx.x];
@@ -247,48 +272,38 @@ __global__ void __launch_bounds__(kIntThreads) k_gauss_b(IntegrateArgs a) {
   const double dt = S.dt;
   const double inv = (xi_old == 0.0) ? 1.0 : 1.0 / (1.0 + xi * 0.5 * dt);
   const double cv = dt - xi * 0.5 * dt * dt;
-  double mv2 = 0;
+  Terms<1, kT> sum;
 #pragma unroll
-  for (int j0 = 0; j0 < kIntPer; j0 += kIntGroup) {
-    GaussIn g[kIntGroup];
-    float4 p[kIntGroup];
-#pragma unroll
-    for (int j = 0; j < kIntGroup; ++j) {
-      const uint32_t t = threadIdx.x + (j0 + j) * kIntThreads;
-      if (t < m.n) {
-        gauss_load(a, S, m.i0 + t, g[j]);
-        p[j] = a.r[m.i0 + t];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kIntGroup; ++j) {
-      const uint32_t t = threadIdx.x + (j0 + j) * kIntThreads;
-      if (t < m.n) {
-        const uint32_t i = m.i0 + t;
-        double A[3];
-        gauss_A(S, g[j], hx, A);
-        const double v[3] = {A[0] * inv, A[1] * inv, A[2] * inv};
-        const double cf = 0.5 * dt * dt * (double)g[j].minv;
-        float4 q = p[j];
-        q.x = (float)((double)q.x + v[0] * cv + (double)g[j].F.x * cf);
-        q.y = (float)((double)q.y + v[1] * cv + (double)g[j].F.y * cf);
-        q.z = (float)((double)q.z + v[2] * cv + (double)g[j].F.z * cf);
-        if (a.wrap) wrap3(S, q);
-        a.r[i] = q;
-        if (a.vd) {
-          store_vd(a, S, i, v);
-          mv2 = add_mv2(mv2, g[j].mass, v[0], v[1], v[2]);
-        } else {
-          const float4 vf = make_float4((float)v[0], (float)v[1], (float)v[2], 0.f);
-          a.v[i] = vf;
-          mv2 = add_mv2(mv2, g[j].mass, vf.x, vf.y, vf.z);
-        }
+  for (int j = 0; j < kIntAtoms / kT; ++j) {
+    const uint32_t t = threadIdx.x + j * kT;
+    if (t < m.n) {
+      const uint32_t i = m.i0 + t;
+      GaussIn g;
+      gauss_load(a, S, i, g);
+      float4 q = a.r[i];
+      double A[3];
+      gauss_A(S, g, hx, A);
+      const double v[3] = {A[0] * inv, A[1] * inv, A[2] * inv};
+      const double cf = 0.5 * dt * dt * (double)g.minv;
+      q.x = (float)__fma_rn((double)g.F.x, cf, __fma_rn(v[0], cv, (double)q.x));
+      q.y = (float)__fma_rn((double)g.F.y, cf, __fma_rn(v[1], cv, (double)q.y));
+      q.z = (float)__fma_rn((double)g.F.z, cf, __fma_rn(v[2], cv, (double)q.z));
+      if (a.wrap) wrap3(S, q);
+      a.r[i] = q;
+      if (a.vd) {
+        store_vd(a, S, i, v);
+        sum.add(0, mv2_term(g.mass, v[0], v[1], v[2]));
+      } else {
+        const float4 vf = make_float4((float)v[0], (float)v[1], (float)v[2], 0.f);
+        a.v[i] = vf;
+        sum.add(0, mv2_term(g.mass, vf.x, vf.y, vf.z));
       }
     }
   }
-  double s[1] = {mv2}, tot[1];
-  block_sum<1>(s, red);
-  if (sys_total<1>(s, a.partials, blockIdx.x, S.blk0, S.nblk, &sc.counter[2], tot, red)) {
+  sum.gather();
+  double tot[1];
+  block_sum<1>(sum.s, red);
+  if (sys_total<1>(sum.s, a.partials, blockIdx.x, S.blk0, S.nblk, &sc.counter[2], tot, red)) {
     sc.mv2 = tot[0];
     sc.xi_old = xi;  // every other block of this system has finished reading xi_old
     if (!isfinite(tot[0])) atomicOr(&a.status[m.sys], kStatusNonFinite);
@@ -315,7 +330,7 @@ __global__ void __launch_bounds__(kIntThreads) k_mv2(IntegrateArgs a) {
     const uint32_t i = m.i0 + t;
     double v[3];
     load_v(a, S, i, v);
-    s[0] = add_mv2(s[0], a.mass[i], v[0], v[1], v[2]);
+    s[0] = __dadd_rn(s[0], mv2_term(a.mass[i], v[0], v[1], v[2]));
   }
   double tot[1];
   block_sum<1>(s, red);
@@ -511,7 +526,7 @@ __global__ void __launch_bounds__(kIntThreads) k_gather_state(GatherArgs g) {
   if (q.src < 0) {  // a new system starts from zeros, as a new engine's arrays do
     const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
     for (uint32_t t = threadIdx.x; t < m.n; t += kIntThreads) {
-      const uint32_t off = m.k * kIntAtoms + t, i = m.i0 + t;
+      const uint32_t i = m.i0 + t, off = i - g.sys[m.sys].atom0;
       g.r[i] = z4;
       g.F0[i] = z4;
       g.F1[i] = z4;
@@ -528,8 +543,8 @@ __global__ void __launch_bounds__(kIntThreads) k_gather_state(GatherArgs g) {
     return;
   }
   for (uint32_t t = threadIdx.x; t < m.n; t += kIntThreads) {
-    const uint32_t off = m.k * kIntAtoms + t;  // atom within its system
-    const uint32_t i = m.i0 + t, o = q.o_atom0 + off;
+    const uint32_t i = m.i0 + t, off = i - g.sys[m.sys].atom0;  // atom within its system
+    const uint32_t o = q.o_atom0 + off;
     g.r[i] = g.o_r[o];
     g.F0[i] = (q.fb0 ? g.o_F1 : g.o_F0)[o];
     g.F1[i] = (q.fb1 ? g.o_F1 : g.o_F0)[o];
@@ -571,10 +586,11 @@ void make_block_map(const uint32_t *natoms, uint32_t nsys, BlockMap *map, uint32
   for (uint32_t s = 0; s < nsys; ++s) {
     blk0[s] = b;
     nblk[s] = blocks_for(natoms[s]);
+    const uint32_t per = kIntAtoms;
     for (uint32_t k = 0; k < nblk[s]; ++k) {
-      const uint32_t i0 = atom0 + k * kIntAtoms;
-      const uint32_t n = natoms[s] - k * kIntAtoms;
-      map[b++] = BlockMap{s, i0, n < (uint32_t)kIntAtoms ? n : (uint32_t)kIntAtoms, k};
+      const uint32_t i0 = atom0 + k * per;
+      const uint32_t n = natoms[s] - k * per;
+      map[b++] = BlockMap{s, i0, n < per ? n : per, k};
     }
     atom0 += natoms[s];
   }
@@ -589,7 +605,9 @@ void make_block_map(const uint32_t *natoms, uint32_t nsys, BlockMap *map, uint32
 
 cudaError_t launch_vv(const IntegrateArgs &a, cudaStream_t s) {
   if (!a.nblocks) return cudaSuccess;
-  return launch_pdl(k_vv, dim3(a.nblocks), dim3(kIntThreads), 0, s, a);
+  return a.nblocks <= kIntWideBlocks
+             ? launch_pdl(k_vv<kIntAtoms>, dim3(a.nblocks), dim3(kIntAtoms), 0, s, a)
+             : launch_pdl(k_vv<kIntThreads>, dim3(a.nblocks), dim3(kIntThreads), 0, s, a);
 }
 cudaError_t launch_wrap(const IntegrateArgs &a, cudaStream_t s) { PB_LAUNCH(k_wrap, a); }
 cudaError_t launch_mv2(const IntegrateArgs &a, cudaStream_t s) { PB_LAUNCH(k_mv2, a); }
@@ -600,8 +618,11 @@ cudaError_t launch_scale(const IntegrateArgs &a, const double *f, cudaStream_t s
 
 cudaError_t launch_gauss(const IntegrateArgs &a, cudaStream_t s) {
   if (!a.nblocks) return cudaSuccess;
-  cudaError_t e = launch_pdl(k_gauss_a, dim3(a.nblocks), dim3(kIntThreads), 0, s, a);
-  if (e == cudaSuccess) e = launch_pdl(k_gauss_b, dim3(a.nblocks), dim3(kIntThreads), 0, s, a);
+  const bool wide = a.nblocks <= kIntWideBlocks;
+  const dim3 nb(a.nblocks), nt(wide ? kIntAtoms : kIntThreads);
+  cudaError_t e = launch_pdl(wide ? k_gauss_a<kIntAtoms> : k_gauss_a<kIntThreads>, nb, nt, 0, s, a);
+  if (e == cudaSuccess)
+    e = launch_pdl(wide ? k_gauss_b<kIntAtoms> : k_gauss_b<kIntThreads>, nb, nt, 0, s, a);
   return e;
 }
 

@@ -13,9 +13,10 @@
 //   key    uint32[N]   packed cell key of each atom: cell0 + rank(x,y) * nz + z
 //   start  uint32[C+1] first sorted slot of each packed cell (C = all cells)
 //   pid    uint32[N]   particle id at each sorted slot (cudaCutoffBlock::pid)
-//   slot   uint32[N]   sorted slot of each particle (inverse of pid)
+//   slot   uint32[N]   sorted slot of each particle (inverse of pid); only the
+//          allocation-free build writes it
 //   rs     float4[N]   sorted positions, w = type id bits (cudaSortedPositions::r_s)
-//   xs, ys, zs float, ts uint32 [M]  SoA mirrors of rs; system s at mirror0(s) + k,
+//   xs, ys, zs float, ts uint32 [M]  SoA mirrors of rs (half-shell kernel only); system s at mirror0(s) + k,
 //          mirror0 a multiple of 4 (M = sum of the systems' sizes rounded up to 4, + 4)
 // Cell keys order the (x, y) columns of a box along a Morton (Z-order) curve and
 // keep z fastest, so the three z-adjacent cells of a column are contiguous.
@@ -63,7 +64,8 @@ struct CellBufs {
   uint32_t N;
   uint32_t ncells;           // packed cells over all systems
   uint32_t *key, *within, *count, *start, *tilesum;
-  uint32_t *pid_tmp, *pid, *slot;
+  uint32_t *pid_tmp, *pid;
+  uint32_t *slot;            // nullptr: not written
   // two-kernel build (bucket == nullptr: the six-kernel counting sort)
   uint32_t *bucket;          // per cell, bucket_cap member ids in ticket order
   uint32_t bucket_cap;       // at least 32
