@@ -369,8 +369,7 @@ int pb_batch_get(pb_batch *b, uint32_t sys, int field, void *host, size_t bytes)
   const int rc = field_slice(b, sys, field, &p, &need, false);
   if (rc) return rc;
   if (bytes != need) return fail(b, PB_ERR_ARG, "size mismatch for field");
-  B_CUDA(cudaMemcpyAsync(host, p, need, cudaMemcpyDeviceToHost, b->e.stream));
-  B_CUDA(cudaStreamSynchronize(b->e.stream));
+  B_CUDA(engine_read(b->e, host, p, need));
   return PB_OK;
 }
 

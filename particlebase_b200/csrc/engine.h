@@ -141,6 +141,8 @@ int engine_force(Engine &e, bool energy);
 int engine_evolve(Engine &e, int mode, int wrap);
 int engine_wrap(Engine &e);
 int engine_step(Engine &e, int mode);
+// Copies device memory to a host buffer after the work issued so far, and waits.
+cudaError_t engine_read(Engine &e, void *host, const void *dev, size_t bytes);
 // Device scratch from the engine's pool, on its stream (stream-ordered).
 cudaError_t engine_alloc_bytes(Engine &e, void **p, size_t bytes);
 void engine_free_bytes(Engine &e, void *p);

@@ -428,8 +428,7 @@ int pb_md_get(pb_md *h, int field, void *host, size_t bytes) {
     }
     default: return PB_ERR_NOTFOUND;
   }
-  H_CUDA(cudaMemcpyAsync(host, src, need, cudaMemcpyDeviceToHost, e.stream));
-  H_CUDA(cudaStreamSynchronize(e.stream));
+  H_CUDA(engine_read(e, host, src, need));
   return PB_OK;
 }
 
