@@ -284,6 +284,7 @@ __global__ void __launch_bounds__(256) k_canon(CellBufs b) {
 
 constexpr int kTileShift = 6;  // 64 cells per k_canon_tiles block
 constexpr int kTileThreads = 256;
+constexpr uint32_t kSMs = 148;
 constexpr int kCanonPer = 1;   // staged slots a k_canon_tiles thread loads at once (1
                                // measured fastest: 41.6 us, against 42.1 us for 2, 45.9 us for 4)
 
@@ -399,17 +400,24 @@ __device__ __forceinline__ const uint32_t *members(const CellBufs &b, uint32_t k
 // gathers members (id, order key, cell) with independent loads, then ranks
 // its members within their cells and writes them.  Other tiles take one
 // warp per two cells.
-__global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
+// kT threads, kMin blocks per SM.  With 256 threads a tile of 1,000 members takes
+// four to five rounds, which many tiles on an SM hide and few do not, so the
+// fewer tiles there are the more threads each takes.  Whole steps: 4,000 atoms (4
+// tiles) 30.7 -> 26.3 us with 1,024 threads, 131,072 atoms (125) 65.4 -> 57.2;
+// 262,144 (267) 110.0 -> 101.0 with 512, three per SM; 500,000 (550) 170.5 ->
+// 164.1 with 512, four per SM; 1M atoms (1,158) 345.3 with 256, 348.5 with 512.
+template <int kT, int kMin>
+__global__ void __launch_bounds__(kT, kMin) k_canon_tiles(CellBufs b) {
   pdl_enter();
   extern __shared__ __align__(16) unsigned char tsm[];
-  __shared__ uint32_t red[kTileThreads / 32];
+  __shared__ uint32_t red[kT / 32];
   __shared__ uint32_t cst[(1 << kTileShift) + 1];  // tile-local starts, then the total
   __shared__ uint32_t wtot, nmax;
   __shared__ bool is_last;
   const uint32_t t = blockIdx.x, c0 = t << kTileShift;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t acc = 0;
-  for (uint32_t k = threadIdx.x; k < t; k += kTileThreads) acc += b.tcount[k];
+  for (uint32_t k = threadIdx.x; k < t; k += kT) acc += b.tcount[k];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) red[warp] = acc;
@@ -430,7 +438,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
   __syncthreads();
   uint32_t base = 0;
 #pragma unroll
-  for (int w = 0; w < kTileThreads / 32; ++w) base += red[w];
+  for (int w = 0; w < kT / 32; ++w) base += red[w];
   if (threadIdx.x < (1u << kTileShift)) {
     const uint32_t loc = (warp == 1 ? wtot : 0u) + incl - n;
     cst[threadIdx.x] = loc;
@@ -450,11 +458,11 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
     uint8_t *scl = reinterpret_cast<uint8_t *>(szk + b.tile_atoms);
     // gather: slot j of the tile -> (cell k, member j - cst[k]); a thread's
     // slots are taken kCanonPer at a time, each load step issued for all
-    for (uint32_t j0 = threadIdx.x; j0 < T; j0 += kCanonPer * kTileThreads) {
+    for (uint32_t j0 = threadIdx.x; j0 < T; j0 += kCanonPer * kT) {
       uint32_t me[kCanonPer];
 #pragma unroll
       for (int u = 0; u < kCanonPer; ++u) {
-        const uint32_t j = j0 + (uint32_t)u * kTileThreads;
+        const uint32_t j = j0 + (uint32_t)u * kT;
         if (j >= T) break;
         uint32_t lo = 0, hi = 1u << kTileShift;  // largest k with cst[k] <= j
         while (hi - lo > 1) {
@@ -466,7 +474,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
       }
 #pragma unroll
       for (int u = 0; u < kCanonPer; ++u) {
-        const uint32_t j = j0 + (uint32_t)u * kTileThreads;
+        const uint32_t j = j0 + (uint32_t)u * kT;
         if (j >= T) break;
         sid[j] = me[u];
         szk[j] = z_key(b.r[me[u]].z);
@@ -474,12 +482,12 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
     }
     __syncthreads();
     // rank within the cell by (z, particle id), then write
-    for (uint32_t j0 = threadIdx.x; j0 < T; j0 += kCanonPer * kTileThreads) {
+    for (uint32_t j0 = threadIdx.x; j0 < T; j0 += kCanonPer * kT) {
       float4 p[kCanonPer];
       uint32_t ty[kCanonPer], sy[kCanonPer];
 #pragma unroll
       for (int u = 0; u < kCanonPer; ++u) {
-        const uint32_t j = j0 + (uint32_t)u * kTileThreads;
+        const uint32_t j = j0 + (uint32_t)u * kT;
         if (j >= T) break;
         const uint32_t me = sid[j];
         p[u] = b.r[me];
@@ -488,7 +496,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
       }
 #pragma unroll
       for (int u = 0; u < kCanonPer; ++u) {
-        const uint32_t j = j0 + (uint32_t)u * kTileThreads;
+        const uint32_t j = j0 + (uint32_t)u * kT;
         if (j >= T) break;
         const uint32_t k = scl[j], lo = cst[k], hi = cst[k + 1];
         const uint32_t me = sid[j], kz = szk[j];
@@ -503,7 +511,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
     }
   } else {
     // one warp per two cells, 16 cells per round
-    for (uint32_t r = 0; r < (1u << kTileShift); r += 2 * (kTileThreads / 32)) {
+    for (uint32_t r = 0; r < (1u << kTileShift); r += 2 * (kT / 32)) {
       const uint32_t k0 = r + 2 * (uint32_t)warp;
       const uint32_t ca = c0 + k0;
       if (ca >= b.ncells) break;
@@ -538,7 +546,7 @@ __global__ void __launch_bounds__(kTileThreads, 8) k_canon_tiles(CellBufs b) {
   }
   __syncthreads();
   if (is_last) {
-    for (uint32_t k = threadIdx.x; k < b.ntile; k += kTileThreads) b.tcount[k] = 0u;
+    for (uint32_t k = threadIdx.x; k < b.ntile; k += kT) b.tcount[k] = 0u;
     if (threadIdx.x == 0) {
       b.ctl[0] = 0u;
       b.ctl[1] = 0u;
@@ -556,11 +564,16 @@ cudaError_t launch_cell_build(const CellBufs &b, cudaStream_t s) {
     cudaError_t e = launch_pdl(k_bin_buckets, dim3((b.N + per_block - 1) / per_block),
                                dim3(kTileThreads), 0, s, b);
     const uint32_t smem = tile_smem(b.tile_atoms);
+    const uint32_t n = b.ntile;
+    const int threads = n <= kSMs ? 1024 : n <= 4 * kSMs ? 512 : 256;
+    auto canon = n <= kSMs       ? k_canon_tiles<1024, 1>
+                 : n <= 3 * kSMs ? k_canon_tiles<512, 3>
+                 : n <= 4 * kSMs ? k_canon_tiles<512, 4>
+                                 : k_canon_tiles<256, 8>;
     if (e == cudaSuccess && smem > 48u * 1024u)
-      e = cudaFuncSetAttribute(k_canon_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem);
+      e = cudaFuncSetAttribute(canon, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess)
-      e = launch_pdl(k_canon_tiles, dim3(b.ntile), dim3(kTileThreads), smem, s, b);
+      e = launch_pdl(canon, dim3(b.ntile), dim3(threads), smem, s, b);
     return e;
   }
   cudaError_t e = launch_pdl(k_bin, dim3(nb), dim3(256), 0, s, b);

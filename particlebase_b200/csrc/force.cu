@@ -754,7 +754,6 @@ template <int NT, bool ENERGY, typename Acc, int kWarps, int MODE>
 __global__ void __launch_bounds__(kWarps * 32,
                                   (NT == 1 && !ENERGY && std::is_same<Acc, float>::value && MODE != kModeSoftCore ? 32 : 24) / kWarps)
     k_force(const __grid_constant__ ForceBufs b) {
-  pdl_enter();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ Stage<NT> d;
   __shared__ uint64_t full;
@@ -762,6 +761,16 @@ __global__ void __launch_bounds__(kWarps * 32,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const ForceItem &it = b.items[blockIdx.x];
   const uint32_t sys = it.sys;
+  // what no kernel of a step writes is read ahead of the wait for the cell build
+  if (warp == 1) {
+    plan_frame<NT>(b, it, d);
+  } else if (warp == 2) {
+    load_lj<NT, MODE>(b, b.sys[sys], d);
+  } else if (threadIdx.x == 0) {
+    mbar_init(&full, 1);
+    mbar_fence_init();
+  }
+  pdl_enter();
   if (b.steps_left != nullptr && b.steps_left[sys] == 0) {
     // a system whose step budget is spent keeps its state
     if (ENERGY && threadIdx.x < 4) b.partials[(size_t)blockIdx.x * 4 + threadIdx.x] = 0.0;
@@ -775,16 +784,8 @@ __global__ void __launch_bounds__(kWarps * 32,
   uint32_t *tab = reinterpret_cast<uint32_t *>(smem_raw + (size_t)slots * slot_bytes(NT)) +
                   warp * (warp_bytes(NT) / 4);
   if (warp == 0) {
-    if (lane == 0) {
-      mbar_init(&full, 1);
-      mbar_fence_init();
-    }
     __syncwarp();
     plan_stage<NT>(b, it, d, E, &full);
-  } else if (warp == 1) {
-    plan_frame<NT>(b, it, d);
-  } else if (warp == 2) {
-    load_lj<NT, MODE>(b, b.sys[sys], d);
   }
   __syncthreads();
   if (!d.overflow) {
