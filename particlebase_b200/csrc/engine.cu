@@ -966,11 +966,12 @@ int engine_make_nlist(Engine &e) {
     // expected row length at the system's density, with headroom
     const double vol = (double)g.L[0] * g.L[1] * g.L[2];
     const double expect = N / vol * 4.18879020478639 * rl * rl * rl;
-    const uint32_t cap = ((uint32_t)(1.5 * expect) + 32u + 7u) & ~7u;
+    const uint32_t lanes = nlist_lanes(e.N);
+    const uint32_t cap = ((uint32_t)(1.45 * expect / lanes) + 14u + 1u) & ~1u;
     const uint32_t nb = nlist_blocks(N);
     const uint32_t item0[2] = {0u, nb};
-    bool ok = dalloc(e, &e.nl_idx, (size_t)cap * N) == cudaSuccess &&
-              dalloc(e, &e.nl_cnt, N) == cudaSuccess && dalloc(e, &e.nl_atom, N) == cudaSuccess &&
+    bool ok = dalloc(e, &e.nl_idx, (size_t)cap * lanes * N) == cudaSuccess &&
+              dalloc(e, &e.nl_cnt, (size_t)lanes * N) == cudaSuccess && dalloc(e, &e.nl_atom, N) == cudaSuccess &&
               dalloc(e, &e.nl_max, 1) == cudaSuccess && dalloc(e, &e.nl_r0, N) == cudaSuccess &&
               dalloc(e, &e.nl_rl, N) == cudaSuccess &&
               dalloc(e, &e.nl_partials, (size_t)4 * nb) == cudaSuccess &&
@@ -1000,7 +1001,7 @@ int engine_make_nlist(Engine &e) {
     // build raised is cleared; the rebuilt list is complete)
     dfree(e, e.nl_idx);
     const uint32_t cap = (mx + mx / 4 + 7u) & ~7u;
-    if (dalloc(e, &e.nl_idx, (size_t)cap * N) != cudaSuccess) {
+    if (dalloc(e, &e.nl_idx, (size_t)cap * nlist_lanes(e.N) * N) != cudaSuccess) {
       free_nlist(e);
       return fail(e, PB_ERR_OOM, "neighbour list allocation failed");
     }
@@ -1014,19 +1015,22 @@ int engine_make_nlist(Engine &e) {
 
 int engine_nlist_info(Engine &e, double out[3]) {
   if (!e.nl_on || !e.nl_built) return fail(e, PB_ERR_STATE, "no neighbour list");
-  std::vector<uint32_t> cnt(e.N);
-  E_CUDA(cudaMemcpyAsync(cnt.data(), e.nl_cnt, sizeof(uint32_t) * e.N, cudaMemcpyDeviceToHost,
-                         e.stream));
+  const uint32_t lanes = nlist_lanes(e.N);
+  std::vector<uint32_t> cnt((size_t)lanes * e.N);
+  E_CUDA(cudaMemcpyAsync(cnt.data(), e.nl_cnt, sizeof(uint32_t) * cnt.size(),
+                         cudaMemcpyDeviceToHost, e.stream));
   E_CUDA(cudaStreamSynchronize(e.stream));
   double sum = 0;
   uint32_t mx = 0;
-  for (uint32_t v : cnt) {
-    sum += v;
-    mx = std::max(mx, v);
+  for (size_t s = 0; s < cnt.size(); s += lanes) {
+    uint32_t row = 0;
+    for (uint32_t l = 0; l < lanes; ++l) row += cnt[s + l];
+    sum += row;
+    mx = std::max(mx, row);
   }
   out[0] = e.N ? sum / e.N : 0.0;
   out[1] = mx;
-  out[2] = e.nl_cap;
+  out[2] = (double)e.nl_cap * lanes;
   return PB_OK;
 }
 

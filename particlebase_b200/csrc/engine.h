@@ -100,7 +100,7 @@ struct Engine {
   // force calls use the list and whole steps skip the cell-list build
   bool nl_on = false, nl_built = false;
   float nl_skin = 0.f;
-  uint32_t nl_cap = 0;  // entries per row
+  uint32_t nl_cap = 0;  // entries per part of a row (nlist_lanes(N) parts)
   uint32_t *nl_idx = nullptr, *nl_cnt = nullptr, *nl_atom = nullptr, *nl_max = nullptr;
   float4 *nl_r0 = nullptr, *nl_rl = nullptr;
   double *nl_partials = nullptr;

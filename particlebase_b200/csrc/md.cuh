@@ -117,7 +117,7 @@ struct ForceBufs {
 
 // Verlet neighbour list of one system: row s holds the build-time sorted
 // slots of the atoms within the list radius of the atom that sat in slot s
-// when the list was built, column-major (entry k of row s at idx[k * N + s]).
+// when the list was built, in nlist_lanes(N) parts (layout: nlist.cu).
 struct NlistBufs {
   const float4 *r;           // positions, particle order
   const float4 *rs;          // sorted positions (build)
@@ -125,13 +125,13 @@ struct NlistBufs {
   const uint16_t *type;
   const SysDesc *sys;        // the one system
   const LJTable *lj;
-  uint32_t N, cap;           // atoms; entries per row
+  uint32_t N, cap;           // atoms; entries per part of a row
   float rl2;                 // list radius squared (build)
   float skin;                // list radius minus the force cutoff
-  uint32_t *idx, *cnt, *atom;  // rows, row counts, particle of each row
+  uint32_t *idx, *cnt, *atom;  // rows, counts of their parts, particle of each row
   float4 *rl;                // current positions in row order (refreshed every force call)
   float4 *r0;                // positions at the build, row order
-  uint32_t *maxcnt;          // build: largest row count (reset by the caller)
+  uint32_t *maxcnt;          // build: largest count of a part (reset by the caller)
   float4 *F;                 // force output, particle order
   double *partials;          // per-block energy partials (4 doubles per block)
   uint32_t *status;
@@ -153,6 +153,7 @@ cudaError_t launch_nlist_build(const NlistBufs &b, cudaStream_t s);
 // (launch_nlist_force refreshes rl from r before the pair loop)
 cudaError_t launch_nlist_force(const NlistBufs &b, int nt_max, bool energy, bool acc64,
                                cudaStream_t s);
+uint32_t nlist_lanes(uint32_t N);    // parts of a row
 uint32_t nlist_blocks(uint32_t N);  // blocks (energy partials) of launch_nlist_force
 // Pair counts per distance bin over all unordered pairs (g(r)); counts must
 // be zeroed by the caller; rnum <= gr_max_bins().

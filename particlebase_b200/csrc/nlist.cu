@@ -9,14 +9,17 @@
 // only with the list, as testMD4n.cu:175-181 does.
 //
 // Layout.  Instead of CSR (a count pass, a scan and a fill pass), rows have a
-// fixed capacity and are stored column-major: entry k of row s at
-// idx[k * N + s], so the threads of a warp (consecutive rows) read one
-// coalesced line per entry.  Row s belongs to the atom that sat in sorted slot
-// s at the build, and entries are build-time slots too: every force call first
-// copies the current positions into that order (rl), so a warp's atoms are
-// neighbours of one another and the positions they gather sit in a few nearby
-// lines, mostly shared through L1.  The build reports the longest row; the
-// host grows the capacity and rebuilds when a row did not fit.
+// fixed capacity.  L = 1, 2 or 4 lanes share a row (by the number of rows): at the
+// build they take its candidates in turn and each keeps its own part of the row,
+// so no count has to be known to another lane, and the force kernel's lanes read
+// their parts back.  Entry k of lane l of row s is at idx[L (k N + s) + l], so a
+// warp reads one line per entry.  Row s belongs to the atom that sat in sorted slot s at the
+// build, and entries are build-time slots too: every force call first copies the
+// current positions into that order (rl), so a warp's atoms are neighbours of one
+// another and the positions they gather sit in a few nearby lines, mostly shared
+// through L1.  The build reports the longest part of a row; the host grows the
+// capacity and rebuilds when one did not fit.  Both kernels are bound by the
+// latency of dependent loads.
 //
 // Minimum image.  Each component of a pair difference is x_i - x_j, and when
 // that exceeds half the box the coordinate above the box middle is moved down
@@ -33,6 +36,7 @@ namespace {
 
 constexpr int kNlThreads = 256;
 
+
 __device__ __forceinline__ float image_delta(float xi, float xj, float L, float hL) {
   const float d = xi - xj;
   if (d > hL) return (xi - L) - xj;
@@ -44,18 +48,19 @@ __device__ __forceinline__ float round_image(float d, float L, float Linv) {
   return d - L * rintf(d * Linv);
 }
 
-// Row s of the list, built by one thread; returns its length (entries beyond
-// the capacity are counted, not stored).  The three cells z - 1, z, z + 1 of a neighbour column
+// Lane l's part of row s of the list; returns its length (entries beyond the
+// capacity are counted, not stored).  The three cells z - 1, z, z + 1 of a neighbour column
 // are consecutive in sorted order and sorted by z, so each column is one
 // range: a binary search finds its first atom inside the atom's z window,
 // and the scan stops at the first atom above it.  The window half-width
 // shrinks with the atom's distance in x and y from that column, a bound
 // taken with a margin of 10^-3 cell edges (cell membership is decided in
-// FP32).  The column's periodic image is applied as one shift.  A column
+// FP32).  The lanes take the range's atoms in turn.  The column's periodic image
+// is applied as one shift.  A column
 // whose z cells wrap around the box (z = 0 or nz - 1) is scanned cell by
-// cell, with a shift per cell.  Candidates are visited in sorted order, so a
-// row lists its atoms in the same order as a scan of the 27 cells.
-__device__ uint32_t nlist_row(const NlistBufs &b, uint32_t s) {
+// cell, with a shift per cell.  Candidates are visited in sorted order.
+template <uint32_t L>
+__device__ uint32_t nlist_row(const NlistBufs &b, uint32_t s, uint32_t l) {
   const SysDesc &S = b.sys[0];
   const Grid g = S.g;
   const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
@@ -78,7 +83,7 @@ __device__ uint32_t nlist_row(const NlistBufs &b, uint32_t s) {
   auto take = [&](uint32_t t, float qx, float qy, float qz, float sx, float sy, float sz) {
     const float dx = (qx + sx) - p.x, dy = (qy + sy) - p.y, dz = (qz + sz) - p.z;
     if (t != s && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < b.rl2) {
-      if (n < b.cap) b.idx[(size_t)n * b.N + s] = t;
+      if (n < b.cap) b.idx[((size_t)n * b.N + s) * L + l] = t;
       ++n;
     }
   };
@@ -99,13 +104,14 @@ __device__ uint32_t nlist_row(const NlistBufs &b, uint32_t s) {
           const float sz = ze < 0 ? -Lz : (ze >= nz ? Lz : 0.f);
           const uint32_t key2 = kb + (uint32_t)((ze + nz) % nz);
           const uint32_t t1 = b.start[key2 + 1];
-          for (uint32_t t0 = b.start[key2]; t0 < t1; t0 += 4) {
+          for (uint32_t t0 = b.start[key2] + l; t0 < t1; t0 += 4 * L) {
             float4 q[4];  // four candidates per pass, their loads issued together
 #pragma unroll
-            for (int u = 0; u < 4; ++u) q[u] = b.rs[min(t0 + u, t1 - 1)];
+            for (uint32_t u = 0; u < 4; ++u) q[u] = b.rs[min(t0 + u * L, t1 - 1)];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (t0 + u < t1) take(t0 + u, q[u].x, q[u].y, q[u].z, sx, sy, sz);
+            for (uint32_t u = 0; u < 4; ++u)
+              if (t0 + u * L < t1)
+                take(t0 + u * L, q[u].x, q[u].y, q[u].z, sx, sy, sz);
           }
         }
         continue;
@@ -126,30 +132,33 @@ __device__ uint32_t nlist_row(const NlistBufs &b, uint32_t s) {
         }
       }
       bool past = false;
-      for (uint32_t t0 = lo; t0 < hi && !past; t0 += 4) {
+      for (uint32_t t0 = lo + l; t0 < hi && !past; t0 += 4 * L) {
         float4 q[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) q[u] = b.rs[min(t0 + u, hi - 1)];
+        for (uint32_t u = 0; u < 4; ++u) q[u] = b.rs[min(t0 + u * L, hi - 1)];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          past = past || t0 + u >= hi || q[u].z > zhi;
-          if (!past) take(t0 + u, q[u].x, q[u].y, q[u].z, sx, sy, 0.f);
+        for (uint32_t u = 0; u < 4; ++u) {
+          past = past || t0 + u * L >= hi || q[u].z > zhi;
+          if (!past) take(t0 + u * L, q[u].x, q[u].y, q[u].z, sx, sy, 0.f);
         }
       }
     }
   }
-  b.cnt[s] = n;
-  b.atom[s] = i;
-  b.r0[s] = make_float4(p.x, p.y, p.z, 0.0f);
+  b.cnt[s * L + l] = n;
+  if (l == 0) {
+    b.atom[s] = i;
+    b.r0[s] = make_float4(p.x, p.y, p.z, 0.0f);
+  }
   if (n > b.cap) atomicOr(&b.status[0], kStatusNlistOverflow);
   return n;
 }
 
+template <uint32_t L>
 __global__ void __launch_bounds__(kNlThreads) k_nlist_build(NlistBufs b) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  // the longest row goes to one counter: a maximum over the warp first, then
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x, s = u / L;
+  // the longest part goes to one counter: a maximum over the warp first, then
   // one atomic per warp (an atomic per row on one address serialises)
-  const uint32_t n = s < b.N ? nlist_row(b, s) : 0u;
+  const uint32_t n = s < b.N ? nlist_row<L>(b, s, u % L) : 0u;
   const uint32_t wmax = __reduce_max_sync(0xffffffffu, n);
   if ((threadIdx.x & 31) == 0 && wmax > 0) atomicMax(b.maxcnt, wmax);
 }
@@ -157,6 +166,7 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_build(NlistBufs b) {
 // Current positions in row order, so the pair loop gathers from build-time
 // slots (type id bits in w, as in the sorted positions).
 __global__ void __launch_bounds__(kNlThreads) k_nlist_gather(NlistBufs b) {
+  pdl_enter();
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= b.N) return;
   const uint32_t i = b.atom[s];
@@ -164,10 +174,11 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_gather(NlistBufs b) {
   b.rl[s] = make_float4(p.x, p.y, p.z, __int_as_float((int)b.type[i]));
 }
 
-template <int NT, bool ENERGY, typename Acc>
+template <int NT, bool ENERGY, typename Acc, uint32_t L>
 __global__ void __launch_bounds__(kNlThreads) k_nlist_force(NlistBufs b) {
   __shared__ float s2[NT * NT], e24[NT * NT], e4[NT * NT], rc2[NT * NT], ush[NT * NT];
   __shared__ double red[4 * 32];
+  pdl_enter();
   if (threadIdx.x < NT * NT) {
     const LJTable &T = b.lj[0];
     const int k = (threadIdx.x / NT) * T.nt + threadIdx.x % NT;
@@ -181,14 +192,16 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_force(NlistBufs b) {
   const Grid g = b.sys[0].g;
   const float Lx = g.L[0], Ly = g.L[1], Lz = g.L[2];
   const float hx = 0.5f * Lx, hy = 0.5f * Ly, hz = 0.5f * Lz;
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t u0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t s = u0 / L, l = u0 % L;
   Acc pe = 0, pes = 0, vir = 0;
   uint32_t npairs = 0;
+  // (a row's lanes are all below N rows or none is)
   if (s < b.N) {
     const uint32_t i = b.atom[s];
     const float4 p = b.rl[s];
     const int ti = NT == 1 ? 0 : __float_as_int(p.w);
-    const uint32_t n = min(b.cnt[s], b.cap);
+    const uint32_t n = min(b.cnt[u0], b.cap);
     Acc fx = 0, fy = 0, fz = 0;
     // four entries per pass: their row reads, then their position gathers, are
     // issued before any of them is used (memory-level parallelism)
@@ -197,7 +210,7 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_force(NlistBufs b) {
       uint32_t t[kU];
 #pragma unroll
       for (int u = 0; u < kU; ++u)
-        t[u] = k0 + u < n ? __ldg(&b.idx[(size_t)(k0 + u) * b.N + s]) : s;
+        t[u] = k0 + u < n ? __ldg(&b.idx[((size_t)(k0 + u) * b.N + s) * L + l]) : s;
       float4 q[kU];
 #pragma unroll
       for (int u = 0; u < kU; ++u) q[u] = b.rl[t[u]];
@@ -227,12 +240,19 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_force(NlistBufs b) {
         }
       }
     }
-    b.F[i] = make_float4((float)fx, (float)fy, (float)fz, 0.0f);
+    const uint32_t mates = ((1u << L) - 1u) << (threadIdx.x & 31u & ~(L - 1u));
+#pragma unroll
+    for (int o = 1; o < (int)L; o <<= 1) {
+      fx += __shfl_xor_sync(mates, fx, o);
+      fy += __shfl_xor_sync(mates, fy, o);
+      fz += __shfl_xor_sync(mates, fz, o);
+    }
+    if (l == 0) b.F[i] = make_float4((float)fx, (float)fy, (float)fz, 0.0f);
     // has the atom left the skin the list was built with?
     const float4 p0 = b.r0[s];
     const float ex = image_delta(p.x, p0.x, Lx, hx), ey = image_delta(p.y, p0.y, Ly, hy);
     const float ez = image_delta(p.z, p0.z, Lz, hz);
-    if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > 0.25f * b.skin * b.skin)
+    if (l == 0 && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > 0.25f * b.skin * b.skin)
       atomicOr(&b.status[0], kStatusStaleList);
   }
   if (ENERGY) {
@@ -243,27 +263,50 @@ __global__ void __launch_bounds__(kNlThreads) k_nlist_force(NlistBufs b) {
   }
 }
 
+template <int NT, uint32_t L>
+auto pick(bool energy, bool acc64) -> void (*)(NlistBufs) {
+  return energy ? (acc64 ? k_nlist_force<NT, true, double, L> : k_nlist_force<NT, true, float, L>)
+                : (acc64 ? k_nlist_force<NT, false, double, L>
+                         : k_nlist_force<NT, false, float, L>);
+}
+
 template <int NT>
 cudaError_t launch_nt(const NlistBufs &b, bool energy, bool acc64, cudaStream_t s) {
-  const uint32_t nb = nlist_blocks(b.N);
-  k_nlist_gather<<<nb, kNlThreads, 0, s>>>(b);
-  if (energy) {
-    if (acc64) k_nlist_force<NT, true, double><<<nb, kNlThreads, 0, s>>>(b);
-    else k_nlist_force<NT, true, float><<<nb, kNlThreads, 0, s>>>(b);
-  } else {
-    if (acc64) k_nlist_force<NT, false, double><<<nb, kNlThreads, 0, s>>>(b);
-    else k_nlist_force<NT, false, float><<<nb, kNlThreads, 0, s>>>(b);
+  cudaError_t e = launch_pdl(k_nlist_gather, dim3((b.N + kNlThreads - 1) / kNlThreads),
+                             dim3(kNlThreads), 0, s, b);
+  if (e != cudaSuccess) return e;
+  void (*kern)(NlistBufs) = nullptr;
+  switch (nlist_lanes(b.N)) {
+    case 4: kern = pick<NT, 4>(energy, acc64); break;
+    case 2: kern = pick<NT, 2>(energy, acc64); break;
+    default: kern = pick<NT, 1>(energy, acc64); break;
   }
-  return cudaGetLastError();
+  return launch_pdl(kern, dim3(nlist_blocks(b.N)), dim3(kNlThreads), 0, s, b);
 }
 
 }  // namespace
 
-uint32_t nlist_blocks(uint32_t N) { return (N + kNlThreads - 1) / kNlThreads; }
+// Lanes per row.  Few rows leave most warps idle, so each is shared by more lanes;
+// many rows fill the chip, and lanes that share one gather from fewer
+// neighbouring rows.  Step (rebuild every 5) with 1, 2 and 4 lanes: 4,000 atoms
+// 33.6, 23.3, 18.1 us; 32,000 36.1, 25.8, 22.0; 64,000 38.4, 30.3, 31.5; 107,999
+// 41.6, 38.5, 42.6; 200,000 64.6, 68.1, 82.8.  List build with its host read: 4,000
+// atoms 138, 110, 75 us; 107,999 204, 186, 182.
+uint32_t nlist_lanes(uint32_t N) { return N <= 49152u ? 4u : (N <= 131072u ? 2u : 1u); }
+
+uint32_t nlist_blocks(uint32_t N) {
+  const uint32_t rows = kNlThreads / nlist_lanes(N);
+  return (N + rows - 1) / rows;
+}
 
 cudaError_t launch_nlist_build(const NlistBufs &b, cudaStream_t s) {
   if (b.N == 0) return cudaSuccess;
-  k_nlist_build<<<nlist_blocks(b.N), kNlThreads, 0, s>>>(b);
+  const uint32_t nb = nlist_blocks(b.N);
+  switch (nlist_lanes(b.N)) {
+    case 4: k_nlist_build<4><<<nb, kNlThreads, 0, s>>>(b); break;
+    case 2: k_nlist_build<2><<<nb, kNlThreads, 0, s>>>(b); break;
+    default: k_nlist_build<1><<<nb, kNlThreads, 0, s>>>(b); break;
+  }
   return cudaGetLastError();
 }
 

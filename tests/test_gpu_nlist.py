@@ -99,3 +99,34 @@ def test_list_needs_cells_as_wide_as_its_radius(cuda_lib):
         p.makeNList()
     p.useNList(-1.0)  # back to the cell list
     p.calcForce()
+
+
+@pytest.mark.parametrize("n", [257, 49151, 49152, 49153, 131072, 131073])
+def test_list_forces_at_the_edges_of_the_lane_rule(cuda_lib, n):
+    """Lanes per row change with the atom count: list forces against the cell
+    path's on the same positions, and complete rows, on either side."""
+    from particlebase_b200.md import from_system
+    k = max(6, int(np.ceil((n / 4) ** (1 / 3))))
+    s = W.fcc_system(k, 0.8442, 0.72, seed=n)
+    rng = np.random.default_rng(n)
+    keep = np.sort(rng.permutation(s.n)[:n])
+    r = np.mod(s.r[keep] + rng.uniform(-0.1, 0.1, (n, 3)), s.L).astype(np.float32)
+    s.r = np.minimum(r, np.nextafter(np.float32(s.L), np.float32(0))).astype(np.float64)
+    s.v, s.mass, s.types = s.v[keep], s.mass[keep], s.types[keep]
+    p = from_system(s, cell_rmax=2.9)
+    p.calcBlockID()
+    p.calcForce()
+    F = p.get("F")[:, :3].astype(np.float64)
+    p.useNList(0.4)
+    p.makeNList()
+    p.calcForce(energy=True)
+    G = p.get("F")[:, :3].astype(np.float64)
+    assert np.sqrt(((F - G) ** 2).sum() / (F ** 2).sum()) < 1e-6
+    info = p.nlist_info()
+    assert 0 < info["mean"] <= info["max"] <= info["capacity"]
+    pe = p.sums()["pe"]
+    p.useNList(-1.0)
+    p.calcBlockID()
+    p.calcForce(energy=True)
+    assert abs(pe - p.sums()["pe"]) < 1e-6 * abs(pe)
+    assert p.status() == 0
