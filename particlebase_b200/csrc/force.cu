@@ -525,6 +525,7 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
   const int tbt = NT == 1 ? 0 : __float_as_int(pb.w) * NT;
   float2 s2 = make_float2(d.lj.s2[0], d.lj.s2[0]);
   float2 e24 = make_float2(d.lj.e24[0], d.lj.e24[0]);
+  float2 e4 = make_float2(d.lj.e4[0], d.lj.e4[0]);
   uint32_t rca = less_1(d.lj.rc2[0]), rcb = rca;  // bits of rc^2, less one
   float4 l0a, l1a, l0b, l1b;
   if (NT == 2) {
@@ -641,20 +642,20 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
             }
             if (ENERGY) {
               const int ka = ta + tj, kb = tbt + tj;
-              const float2 e4 = make_float2(d.lj.e4[ka], d.lj.e4[kb]);
+              if (NT > 1) e4 = make_float2(d.lj.e4[ka], d.lj.e4[kb]);
               float2 u = __fmul2_rn(__fmul2_rn(e4, sr6), __fadd2_rn(sr6, m1));
               u.x = ina ? u.x : 0.0f;
               u.y = inb ? u.y : 0.0f;
-              const float2 us = make_float2(ina ? u.x - d.lj.ush[ka] : 0.0f,
-                                            inb ? u.y - d.lj.ush[kb] : 0.0f);
+              // (a pair's half share is taken at the end: a power of two)
+              acca.pe += (Acc)u.x;
+              accb.pe += (Acc)u.y;
+              if (NT > 1) {  // one type: from pe and the count, at the end
+                acca.pes += (Acc)(ina ? u.x - d.lj.ush[ka] : 0.0f);
+                accb.pes += (Acc)(inb ? u.y - d.lj.ush[kb] : 0.0f);
+              }
               // f is zero outside the cutoff, where r^2 may be +inf
-              const float2 w = make_float2(ina ? f.x * r2c.x : 0.0f, inb ? f.y * r2c.y : 0.0f);
-              acca.pe += (Acc)(0.5f * u.x);
-              accb.pe += (Acc)(0.5f * u.y);
-              acca.pes += (Acc)(0.5f * us.x);
-              accb.pes += (Acc)(0.5f * us.y);
-              acca.vir += (Acc)(0.5f * w.x);
-              accb.vir += (Acc)(0.5f * w.y);
+              acca.vir += (Acc)(ina ? f.x * r2c.x : 0.0f);
+              accb.vir += (Acc)(inb ? f.y * r2c.y : 0.0f);
               acca.n += (uint32_t)ina + (uint32_t)inb;
             }
           } else {
@@ -686,10 +687,12 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
   if (t == 0 && va) b.F[pi] = make_float4((float)v[0], (float)v[1], (float)v[2], 0.0f);
   if (t == 1 && vb) b.F[pi] = make_float4((float)v[3], (float)v[4], (float)v[5], 0.0f);
   if (ENERGY) {
-    const double e[4] = {warp_sum((double)(acca.pe + accb.pe)),
-                         warp_sum((double)(acca.pes + accb.pes)),
-                         warp_sum((double)(acca.vir + accb.vir)),
-                         (double)warp_sum(acca.n + accb.n)};
+    double e[4] = {warp_sum((double)(acca.pe + accb.pe)), warp_sum((double)(acca.pes + accb.pes)),
+                   warp_sum((double)(acca.vir + accb.vir)), (double)warp_sum(acca.n + accb.n)};
+    if (kPacked) {
+      if (NT == 1) e[1] = e[0] - e[3] * (double)d.lj.ush[0];
+      for (int k = 0; k < 3; ++k) e[k] *= 0.5;
+    }
     if (lane == 0)
       for (int k = 0; k < 4; ++k) ce[k] = e[k];
   }
