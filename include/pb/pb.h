@@ -155,11 +155,12 @@ int pb_md_build_cells(pb_md *h);
 #define PB_FORCE_ENERGY 0x1u
 int pb_md_force(pb_md *h, uint32_t flags);
 /* Failure-detection test hook (no counterpart in the reference): one force
- * call in which the force kernel's producer warps withhold
- * their first hand-off to the consumer warps, with every hand-off wait bounded
- * by `polls` polls of at most 1 us.  The consumers' wait runs out, the CTAs
- * end early, the call returns PB_OK and the status word carries
- * PB_STATUS_WAIT_TIMEOUT; the forces of that call are not meaningful.  The
+ * call in which the force kernel's hand-off never comes (the full-shell
+ * kernel's stage copies are not issued; the half-shell kernel's producer warps
+ * withhold their first buffer), with every wait for it bounded by `polls` polls
+ * of at most 1 us.  The wait runs out, the CTAs end early, the call returns
+ * PB_OK and the status word carries PB_STATUS_WAIT_TIMEOUT; the forces of that
+ * call are not meaningful.  The
  * handle stays usable: the next pb_md_force is complete again. */
 int pb_md_force_wait_test(pb_md *h, uint32_t polls);
 /* cudaParticleVV::clearForce (cudaParticleVV.cu:10-15): F = Fold = 0. */

@@ -894,8 +894,6 @@ int force_smem_limit(int nt) {
   return (nt <= 1 ? 56 : 74) * 1024;
 }
 
-int force_threads() { return 256; }
-
 cudaError_t launch_force_capped(const ForceBufs &b, int nt_max, cudaStream_t s) {
   return launch_mode<kModeCapped>(b, nt_max, s);
 }

@@ -14,10 +14,9 @@ namespace pb {
 namespace {
 
 constexpr int kMaxSeg = 32;     // longest z run of one work item (cells)
-constexpr int kListLen = 40;    // per-lane pair list entries
-constexpr int kCopyBatch = 4;   // stage quads a producer thread loads before storing
+constexpr int kListLen = 40;    // per-lane pair list entries (half-shell kernel)
 constexpr int kChunk = 16;      // candidates a lane tests between list checks
-constexpr int kWinCap = 48;     // clusters (or global-path tasks) per item
+constexpr int kWinCap = 48;     // clusters or tiles (or global-path tasks) per item
 constexpr float kFar = 1e30f;   // pad-slot coordinate: never within range
 constexpr float kNoAtom = -1e30f;  // coordinate of a padded home lane
 
@@ -35,12 +34,6 @@ constexpr int kModeLJ = 0;        // truncated LJ (the MD step)
 constexpr int kModeCapped = 1;    // LJ with r^2 floored at (sigma/2)^2 (steepest descent)
 constexpr int kModeSoftCore = 2;  // f0 cos(pi r / 2 rc) along r (initialAnnealing)
 
-// One stage buffer: X, Y, Z planes and, with more than one type, a type plane.
-struct Planes {
-  float *X, *Y, *Z;
-  uint32_t *T;
-};
-
 // Shared-memory access by 32-bit shared address.
 __device__ __forceinline__ float4 lds_f4(uint32_t a) {
   float4 v;
@@ -50,31 +43,6 @@ __device__ __forceinline__ float4 lds_f4(uint32_t a) {
       : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
       : "r"(a));
   return v;
-}
-
-// Read-only global loads of 16 bytes (the sorted-position mirrors, which no
-// kernel writes while the force kernel runs).
-__device__ __forceinline__ float4 ldg_f4(const float *p) {
-  float4 v;
-  asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p));
-  return v;
-}
-
-__device__ __forceinline__ uint4 ldg_u4(const uint32_t *p) {
-  uint4 v;
-  asm("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-      : "l"(p));
-  return v;
-}
-
-// Stage stores of the producers (ordered before their barrier, which is
-// volatile too).
-__device__ __forceinline__ void sts_f4(uint32_t a, float4 v) {
-  asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z),
-               "f"(v.w));
 }
 
 __device__ __forceinline__ float lds_f32(uint32_t a) {
@@ -93,16 +61,6 @@ __device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
 
 __device__ __forceinline__ void sts_u16(uint32_t a, uint32_t v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
-}
-
-__device__ __forceinline__ uint32_t lds_u32(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void sts_u32(uint32_t a, uint32_t v) {
-  asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 // Position of flat quad u in a warp's quad table: within each chunk of 16,

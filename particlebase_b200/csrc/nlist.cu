@@ -44,10 +44,6 @@ __device__ __forceinline__ float image_delta(float xi, float xj, float L, float 
   return d;
 }
 
-__device__ __forceinline__ float round_image(float d, float L, float Linv) {
-  return d - L * rintf(d * Linv);
-}
-
 // Lane l's part of row s of the list; returns its length (entries beyond the
 // capacity are counted, not stored).  The three cells z - 1, z, z + 1 of a neighbour column
 // are consecutive in sorted order and sorted by z, so each column is one
