@@ -139,6 +139,7 @@ struct NlistBufs {
 
 // Launchers (return cudaError_t of the launch).
 cudaError_t launch_cell_build(const CellBufs &b, cudaStream_t s);
+bool cell_build_small(const CellBufs &b);  // the build is one kernel of one block
 cudaError_t launch_force(const ForceBufs &b, int nt_max, bool energy, bool acc64,
                          int block_threads, cudaStream_t s);
 // Half-shell force (each pair once, fixed-point sums) followed by the

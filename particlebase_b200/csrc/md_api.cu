@@ -266,7 +266,7 @@ int pb_md_profile(pb_md *h, float dt, int mode, uint32_t steps, double ms[3]) {
 int pb_md_cell_build_kernels(pb_md *h, uint32_t *kernels) {
   if (!h || !kernels) return PB_ERR_ARG;
   if (!h->e.cells_ready) return fail(h, PB_ERR_STATE, "setup_cells first");
-  *kernels = h->e.cells_bucket ? 2u : 6u;
+  *kernels = cell_build_small(engine_cbufs(h->e)) ? 1u : (h->e.cells_bucket ? 2u : 6u);
   return PB_OK;
 }
 

@@ -223,7 +223,8 @@ class MDSystem:
                                          C.c_float(max_disp)), "minimize")
 
     def cell_build_kernels(self) -> int:
-        """Kernels one cell build launches (2: bucket build, 6: counting sort)."""
+        """Kernels one cell build launches (1: small system, 2: bucket build, 6: counting
+        sort)."""
         k = C.c_uint32()
         self._ck(self.lib.pb_md_cell_build_kernels(self.h, C.byref(k)), "cell_build_kernels")
         return int(k.value)
