@@ -151,7 +151,8 @@ int pb_md_grid(const pb_md *h, uint32_t n3[3], float len3[3], uint32_t *ncells);
  * cudaCutoffBlock.cu:233-258, cudaSortedPositions.cu:27-30). */
 int pb_md_build_cells(pb_md *h);
 /* cudaParticleMD::calcForce (cudaParticleMD.cu:24-69).  flags: PB_FORCE_ENERGY
- * also accumulates PE, shifted PE and virial (FP64) for pb_md_reduce. */
+ * also accumulates PE, shifted PE and virial (FP64) for pb_md_reduce.  The first
+ * call after pb_md_setup_cells builds the cells if pb_md_build_cells has not. */
 #define PB_FORCE_ENERGY 0x1u
 int pb_md_force(pb_md *h, uint32_t flags);
 /* Failure-detection test hook (no counterpart in the reference): one force

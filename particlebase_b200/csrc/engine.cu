@@ -318,6 +318,7 @@ void free_cells(Engine &e) {
   dfree(e, e.fpartials);
   dfree(e, e.fqueue);
   e.cells_ready = false;
+  e.cells_built = false;
 }
 
 void free_nlist(Engine &e) {
@@ -685,6 +686,7 @@ void choose_cell_build(Engine &e) {
   cudaEventDestroy(b);
   e.cells_bucket = !ok || t[0] <= t[1];
   e.cells_chosen = ok;
+  e.cells_built = ok;
 }
 
 int engine_setup_cells(Engine &e) {
@@ -932,8 +934,13 @@ int engine_build(Engine &e) {
   if (!e.cells_ready) return fail(e, PB_ERR_STATE, "setup_cells first");
   cudaError_t c = launch_cell_build(engine_cbufs(e), e.stream);
   if (c != cudaSuccess) return cuda_fail(e, c, "cell build");
+  e.cells_built = true;
   return PB_OK;
 }
+
+// The force kernels take cell starts and sorted positions as they find them:
+// before the first build these arrays hold whatever the pool last kept there.
+int engine_need_cells(Engine &e) { return e.cells_built ? PB_OK : engine_build(e); }
 
 int engine_use_nlist(Engine &e, float thickness) {
   if (e.nsys != 1) return fail(e, PB_ERR_UNSUPPORTED, "neighbour lists are per single system");
@@ -1077,6 +1084,7 @@ int engine_force(Engine &e, bool energy) {
     e.energy_valid = energy;
     return PB_OK;
   }
+  if (const int rc = engine_need_cells(e)) return rc;
   // every ordered pair (the reference's full shell), or with PB_MD_HALF_SHELL
   // every unordered pair once with exact fixed-point sums
   const bool full = (e.flags & PB_MD_ACC_FP64) != 0 || (e.flags & PB_MD_HALF_SHELL) == 0;
@@ -1139,7 +1147,7 @@ int engine_run(Engine &e, int mode, uint32_t steps) {
     cudaGraph_t g = nullptr;
     const int cur0 = e.cur, last0 = e.last;
     const uint64_t done0 = e.steps_done;
-    const bool fresh0 = e.mv2_fresh;
+    const bool fresh0 = e.mv2_fresh, built0 = e.cells_built;
     E_CUDA(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
     int rc = PB_OK;
     for (int k = 0; k < n && !rc; ++k) rc = engine_step(e, mode);
@@ -1148,6 +1156,7 @@ int engine_run(Engine &e, int mode, uint32_t steps) {
     e.last = last0;
     e.steps_done = done0;
     e.mv2_fresh = fresh0;
+    e.cells_built = built0;
     if (rc) {
       if (g) cudaGraphDestroy(g);
       return rc;
@@ -1171,6 +1180,7 @@ int engine_run(Engine &e, int mode, uint32_t steps) {
     for (; done + 2 <= steps; done += 2) {
       E_CUDA(cudaGraphLaunch(g2, e.stream));
       e.steps_done += 2;
+      e.cells_built = e.cells_built || !e.nl_on;
       e.last = 1 - e.cur;  // two steps: cur is back where it was, F[1 - cur] is the newest
     }
   }
@@ -1181,6 +1191,7 @@ int engine_run(Engine &e, int mode, uint32_t steps) {
       if (rc) return rc;
     }
     E_CUDA(cudaGraphLaunch(g1, e.stream));
+    e.cells_built = e.cells_built || !e.nl_on;
     e.steps_done += 1;
     e.last = e.cur;
     e.cur = 1 - e.cur;
@@ -1299,6 +1310,7 @@ int engine_adjust(Engine &e, const double *v1) {
 int engine_force_softcore(Engine &e, float rc, float f0) {
   if (!engine_ready(e)) return fail(e, PB_ERR_STATE, "need cell, LJ parameters and setup_cells");
   if (!(rc > 0)) return fail(e, PB_ERR_ARG, "soft-core range must be > 0");
+  if (const int err = engine_need_cells(e)) return err;
   int nt = 1;
   for (const auto &P : e.sp) nt = std::max(nt, P.lj.nt);
   ForceBufs b = engine_fbufs(e);

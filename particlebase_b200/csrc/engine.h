@@ -63,7 +63,8 @@ struct Engine {
   LJTable *d_lj = nullptr;
 
   // cell list (after setup_cells)
-  bool cells_ready = false;
+  bool cells_ready = false;  // set up: grids, plans and arrays
+  bool cells_built = false;  // a cell build has been issued since the set-up
   uint32_t ncells = 0;
   uint32_t *key = nullptr, *within = nullptr, *tilesum = nullptr, *count = nullptr,
            *start = nullptr, *pid_tmp = nullptr,

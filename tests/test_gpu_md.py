@@ -494,3 +494,30 @@ def test_wait_timeout_is_reported_and_the_handle_recovers(cuda_lib, po):
     assert p.status() == 0
     Fo, _ = oracle_forces(po, s, p.get("r"))
     assert relrms(p.get("F")[:, :3].astype(np.float64), Fo) < FORCE_RELRMS
+
+
+def test_force_calls_without_a_cell_build(cuda_lib):
+    """A force call may come before the first build of the cells: it builds them (the
+    arrays hold nothing yet), also after a later set-up."""
+    s = perturbed(W.config_c1(), 0.05, 3)
+    want = {}
+    for half in (False, True):
+        p = md(cuda_lib, s, half_shell=half)
+        p.calcBlockID()
+        p.calcForce(energy=True)
+        want["lj"], pe = p.get("F"), p.sums()["pe"]
+        p.calcForceSoftCore(2.0, 10.0)
+        want["soft"] = p.get("F")
+        for first in ("lj", "soft"):
+            q = md(cuda_lib, s, half_shell=half)
+            for _ in range(2):
+                if first == "lj":
+                    q.calcForce(energy=True)
+                    assert q.sums()["pe"] == pe
+                else:
+                    q.calcForceSoftCore(2.0, 10.0)
+                assert np.array_equal(q.get("F"), want[first])
+                assert q.status() == 0
+                q.setupCutoffBlock(2.5)
+            q.close()
+        p.close()
