@@ -144,6 +144,7 @@ int pb_batch_repack(const pb_batch *old, const int32_t *src, const uint32_t *nat
     P.lj_set = Q.lj_set;
     P.r_set = Q.r_set;  // positions are gathered from the old batch
     P.lj_percut = Q.lj_percut;
+    P.type_max = Q.type_max;
     P.m0 = Q.m0;
     P.dt = Q.dt;
     nsc[k] = osc[s];
@@ -381,6 +382,7 @@ int pb_batch_set(pb_batch *b, uint32_t sys, int field, const void *host, size_t 
   if (rc) return rc;
   if (bytes != need) return fail(b, PB_ERR_ARG, "size mismatch for field");
   B_CUDA(cudaMemcpyAsync(p, host, need, cudaMemcpyHostToDevice, b->e.stream));
+  if (field == PB_FIELD_TYPE) engine_note_types(b->e, sys, host);
   if (field == PB_FIELD_MINV) {
     const uint32_t n = b->e.sp[sys].n;
     std::vector<float> mi(n), m(n);

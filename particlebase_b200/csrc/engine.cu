@@ -634,6 +634,7 @@ int engine_import(Engine &e, uint32_t sys, const double *r3, const double *v3, c
   if (flags & 1) return fail(e, PB_ERR_ARG, "mass must be positive");
   if (flags & 2) return fail(e, PB_ERR_ARG, "type id >= 8");
   e.sp[sys].m0 = total / n;
+  e.sp[sys].type_max = 0;
   E_CUDA(cudaMemcpyAsync(e.r + a0, r4.get(), 16 * (size_t)n, cudaMemcpyHostToDevice, e.stream));
   E_CUDA(cudaMemcpyAsync(e.minv + a0, minv.get(), 4 * (size_t)n, cudaMemcpyHostToDevice, e.stream));
   E_CUDA(cudaMemcpyAsync(e.mass + a0, m.get(), 4 * (size_t)n, cudaMemcpyHostToDevice, e.stream));
@@ -1067,10 +1068,31 @@ int engine_gr(Engine &e, float rstep, float rmax, uint64_t *counts, uint32_t *rn
   return PB_OK;
 }
 
+void engine_note_types(Engine &e, uint32_t sys, const void *ids) {
+  const unsigned char *p = (const unsigned char *)ids;
+  uint16_t t, m = 0;
+  for (uint32_t i = 0; i < e.sp[sys].n; ++i) {
+    std::memcpy(&t, p + 2 * (size_t)i, 2);
+    m = std::max(m, t);
+  }
+  e.sp[sys].type_max = m;
+}
+
+// Number of types the force kernel is compiled for.  With one type the kernels take no
+// notice of the ids, which may then be any label; with more they index tables by them.
+static int engine_types(Engine &e, int &nt) {
+  uint32_t most = 0;
+  for (const auto &P : e.sp) {
+    nt = std::max(nt, P.lj.nt);
+    most = std::max(most, P.type_max);
+  }
+  return nt > 1 && most >= (uint32_t)kMaxTypes ? fail(e, PB_ERR_ARG, "type id >= 8") : PB_OK;
+}
+
 int engine_force(Engine &e, bool energy) {
   if (!engine_ready(e)) return fail(e, PB_ERR_STATE, "need cell, LJ parameters and setup_cells");
   int nt = 1;
-  for (const auto &P : e.sp) nt = std::max(nt, P.lj.nt);
+  if (const int err = engine_types(e, nt)) return err;
   if (e.nl_on) {
     if (!e.nl_built) return fail(e, PB_ERR_STATE, "make the neighbour list first");
     cudaError_t c = launch_nlist_force(engine_nbufs(e), nt, energy,
@@ -1137,6 +1159,8 @@ int engine_run(Engine &e, int mode, uint32_t steps) {
   if (!engine_ready(e)) return fail(e, PB_ERR_STATE, "need cell, LJ parameters and setup_cells");
   if (mode != PB_MODE_VV && mode != PB_MODE_GAUSS) return fail(e, PB_ERR_ARG, "bad mode");
   if (mode == PB_MODE_VV && e.vd) return fail(e, PB_ERR_UNSUPPORTED, "VV needs FP32 velocities");
+  int nt = 1;
+  if (const int err = engine_types(e, nt)) return err;  // a captured step does not ask
   std::vector<float> dts(e.nsys);
   for (uint32_t s = 0; s < e.nsys; ++s) dts[s] = e.sp[s].dt;
   if (e.graph_mode != mode || e.graph_dt != dts) engine_drop_graph(e);
@@ -1312,7 +1336,7 @@ int engine_force_softcore(Engine &e, float rc, float f0) {
   if (!(rc > 0)) return fail(e, PB_ERR_ARG, "soft-core range must be > 0");
   if (const int err = engine_need_cells(e)) return err;
   int nt = 1;
-  for (const auto &P : e.sp) nt = std::max(nt, P.lj.nt);
+  if (const int err = engine_types(e, nt)) return err;
   ForceBufs b = engine_fbufs(e);
   b.sc_rc = rc;
   b.sc_f0 = f0;
@@ -1335,7 +1359,7 @@ int engine_minimize(Engine &e, uint32_t iters, float alpha, float max_disp) {
   if (!engine_ready(e)) return fail(e, PB_ERR_STATE, "need cell, LJ parameters and setup_cells");
   if (!(alpha > 0) || !(max_disp > 0)) return fail(e, PB_ERR_ARG, "alpha and max_disp must be > 0");
   int nt = 1;
-  for (const auto &P : e.sp) nt = std::max(nt, P.lj.nt);
+  if (const int err = engine_types(e, nt)) return err;
   for (uint32_t it = 0; it < iters; ++it) {
     int rc = engine_build(e);
     if (rc) return rc;

@@ -26,6 +26,7 @@ struct SysParams {
   double m0 = 1.0;
   float dt = 0.005f;
   bool r_set = false;     // positions imported or set (the cell build may be timed)
+  uint32_t type_max = 0;  // largest type id set beyond what an import accepts (below 8)
   bool periodic = true;   // false: open boundaries (pb_md_setup_cells(periodic = 0))
   std::vector<uint32_t> key_of_ref, ref_of_key;  // reference cell id <-> packed key - cell0
 };
@@ -139,6 +140,8 @@ bool engine_ready(const Engine &e);
 
 int engine_build(Engine &e);
 int engine_force(Engine &e, bool energy);
+// Notes the type ids a caller writes for a system (uint16 per atom).
+void engine_note_types(Engine &e, uint32_t sys, const void *ids);
 int engine_evolve(Engine &e, int mode, int wrap);
 int engine_wrap(Engine &e);
 int engine_step(Engine &e, int mode);

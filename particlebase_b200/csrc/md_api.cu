@@ -451,7 +451,10 @@ int pb_md_set(pb_md *h, int field, const void *host, size_t bytes) {
     case PB_FIELD_F: dst = e.F[e.last]; break;
     case PB_FIELD_FOLD: dst = e.F[1 - e.cur]; break;
     case PB_FIELD_MINV: dst = e.minv; break;
-    case PB_FIELD_TYPE: dst = e.type; break;
+    case PB_FIELD_TYPE:
+      dst = e.type;
+      engine_note_types(e, 0, host);
+      break;
     default: return fail(h, PB_ERR_ARG, "field is read-only");
   }
   if (!dst) return fail(h, PB_ERR_STATE, "field not allocated for this handle");

@@ -521,3 +521,47 @@ def test_force_calls_without_a_cell_build(cuda_lib):
                 q.setupCutoffBlock(2.5)
             q.close()
         p.close()
+
+
+@pytest.mark.parametrize("half", [False, True])
+def test_type_ids_beyond_the_tables(cuda_lib, half):
+    """Ids of 8 and more may label the atoms of a one-type system; with more types they
+    would index past the parameter tables, and force calls are refused."""
+    from particlebase_b200._lib import PBError
+    from particlebase_b200.batch import Batch
+    s = perturbed(W.config_c1(), 0.05, 3)
+    p = md(cuda_lib, s, half_shell=half)
+    p.calcBlockID()
+    p.calcForce()
+    F = p.get("F")
+    labels = (np.arange(s.n) % 65536).astype(np.uint16)
+    p.set("type", labels)
+    p.calcBlockID()
+    p.calcForce()
+    assert np.array_equal(p.get("F"), F) and np.array_equal(p.get("type"), labels)
+    p.setLJparams(np.tile([1.0, 1.0], 4), 2)
+    for call in (p.calcForce, lambda: p.calcForceSoftCore(2.0, 1.0), lambda: p.minimize(1),
+                 lambda: p.run(0.005, 2)):
+        with pytest.raises(PBError) as e:
+            call()
+        assert e.value.code == 1
+    p.set("type", labels % 2)
+    p.calcBlockID()
+    p.calcForce()
+    assert np.array_equal(p.get("F"), F)  # both types alike
+    p.run(0.005, 2)
+    p.set("type", labels)
+    with pytest.raises(PBError):
+        p.run(0.005, 2)  # the captured steps are not replayed either
+    p.close()
+    two = W.kob_andersen_random(2000, 1.2, 0.8, seed=7)
+    b = Batch.from_systems([s, two], half_shell=half)
+    b.set(1, "type", np.full(two.n, 8))
+    with pytest.raises(PBError):
+        b.force()
+    again = b.repack([1, 0])
+    with pytest.raises(PBError):
+        again.force()
+    again.set(0, "type", two.types)
+    again.force()
+    assert np.array_equal(again.get(1, "F"), F)
