@@ -191,11 +191,14 @@ __device__ __forceinline__ void global_range(const float4 *__restrict__ P, uint3
 
 // 0 < r2 < rc2 by one unsigned comparison: floats that are not negative order
 // as their bits, r2 = 0 wraps to the largest value and NaNs lie above every rc2.
+// The bound of a pair that does not interact (rc2 = 0) is 0: nothing lies below.
 __device__ __forceinline__ bool inside(float r2, uint32_t rc2_less_1) {
   return __float_as_uint(r2) - 1u < rc2_less_1;
 }
 
-__device__ __forceinline__ uint32_t less_1(float rc2) { return __float_as_uint(rc2) - 1u; }
+__device__ __forceinline__ uint32_t less_1(float rc2) {
+  return rc2 > 0.0f ? __float_as_uint(rc2) - 1u : 0u;
+}
 
 // D = A B + C of one m16n8k8 product, fp16 operands and FP32 sums.
 __device__ __forceinline__ void mma_16x8x8(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b,
@@ -248,7 +251,8 @@ __device__ __forceinline__ void load_lj(const ForceBufs &b, const SysDesc &S, St
   float rc2max = 0.f;
   for (int t = lane; t < NT * NT; t += 32) {
     const int k = t / NT * T.nt + t % NT;
-    const float rc2 = fminf(T.rc2[k], most);
+    // (a cutoff that is not a number is none; the soft core has its own range)
+    const float rc2 = MODE == kModeSoftCore || T.rc2[k] > 0.0f ? fminf(T.rc2[k], most) : 0.0f;
     d.lj.s2[t] = T.s2[k];
     d.lj.e24[t] = T.e24[k];
     d.lj.e4[t] = T.e4[k];

@@ -121,3 +121,48 @@ def test_non_finite_atoms_leave_the_others_alone(cuda_lib):
     s.r, s.types = s.r[keep], s.types[keep]
     F, _ = all_pairs(s)
     assert np.sqrt(((got[keep] - F) ** 2).sum()) < BAR * np.sqrt((F ** 2).sum())
+
+
+def pair_sums(s):
+    """Forces, and the sums over unordered pairs of the energy, the energy less its value
+    at the cutoff, and F . r; the last is the number of ordered pairs inside the cutoff."""
+    d = s.r[:, None] - s.r[None]
+    d -= s.L * np.round(d / s.L)
+    r2 = (d ** 2).sum(-1)
+    sig, eps, rc = np.moveaxis(s.lj[s.types[:, None], s.types[None]], -1, 0)
+    near = (r2 < rc * rc) & (r2 > 0)
+    r2, rc2 = np.where(near, r2, 1.0), np.where(near, rc * rc, 1.0)
+    s6, c6 = (sig * sig / r2) ** 3, (sig * sig / rc2) ** 3
+    fr = np.where(near, 24 * eps * s6 * (2 * s6 - 1), 0.0)
+    u = np.where(near, 4 * eps * s6 * (s6 - 1), 0.0)
+    us = np.where(near, u - 4 * eps * c6 * (c6 - 1), 0.0)
+    return ((fr / r2)[..., None] * d).sum(1), u.sum() / 2, us.sum() / 2, fr.sum() / 2, near.sum()
+
+
+@pytest.mark.parametrize("acc64", [False, True])
+@pytest.mark.parametrize("eps", [1.0, 0.0])
+@pytest.mark.parametrize("ntypes", [2, 3, 5, 8])
+def test_pairs_that_do_not_interact(cuda_lib, ntypes, eps, acc64):
+    """A cutoff of zero switches a pair of types off, whatever its epsilon: no force, no
+    energy, no virial and no pair counted, in dynamics and in the relaxation force (which
+    caps no pair here: none is closer than half a sigma)."""
+    from particlebase_b200.md import from_system
+    s = system((9.0, 10.5, 16.0), 900, ntypes, 20 + ntypes)
+    for a, b in ((0, 0), (0, ntypes - 1), (ntypes - 1, 0)):
+        s.lj[a, b] = s.lj[a, b, 0], eps, 0.0
+    F, *want = pair_sums(s)
+    scale = np.sqrt((F ** 2).sum())
+    p = from_system(s, fp64_forces=acc64)
+    p.calcBlockID()
+    for energy in (False, True):
+        p.calcForce(energy=energy)
+        got = p.get("F")[:, :3].astype(np.float64)
+        assert np.sqrt(((got - F) ** 2).sum()) < BAR * scale
+    e = p.sums()
+    for k, w in zip(("pe", "pe_shift", "virial"), want):
+        assert abs(e[k] - w) < BAR * max(abs(w), 1.0), k
+    assert p.pair_stats()["nin"] == want[3]
+    p.minimize(1)
+    got = p.get("F")[:, :3].astype(np.float64)
+    assert np.sqrt(((got - F) ** 2).sum()) < BAR * scale
+    assert p.status() == 0
