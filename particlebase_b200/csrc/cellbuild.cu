@@ -7,9 +7,10 @@
 // (kernelfuncs.cu:807-932).  The cell of each atom is computed with the same
 // FP32 arithmetic as calcBID_F4, so cell membership is bit-identical; the
 // within-cell order is canonical -- ascending z, ties by particle id -- instead
-// of the reference's history-dependent order.  Because the cell index is a
-// monotone function of z, every (x, y) column of cells is then sorted by z,
-// which the force kernel uses to cut z windows by binary search.
+// of the reference's history-dependent order.  Below the top of the box the cell
+// index is a monotone function of z, so every (x, y) column of cells is then
+// sorted by z, which the force kernels use to cut z windows; atoms more than a
+// cell above the top are filed in cell 0, after the atoms that belong there.
 //
 // Two-kernel build (the engines):
 //   k_bin_buckets  read r (16 B/atom); write key and the atom's id into its

@@ -406,6 +406,36 @@ __device__ __forceinline__ void plan_frame(const ForceBufs &b, const ForceItem &
   }
 }
 
+// Opens the z windows of an item whose staged columns are not all sorted by z (one warp).
+// Cells are sorted, and so are runs of them, except that cell 0 also takes the atoms more
+// than a cell above the top of the box (open boundaries, or positions not wrapped); an
+// image joins its run at the other two seams.  The atoms on either side of a seam are read
+// from global memory, so that no other warp waits and nothing is kept for the tiles.
+template <int NT>
+__device__ __forceinline__ void check_order(const ForceBufs &b, const ForceItem &it, Stage<NT> &d) {
+  const int lane = threadIdx.x & 31, seam = lane / 9;
+  const Grid &g = b.sys[it.sys].g;
+  const int z0 = it.z0, z1 = it.z1, nz = g.n[2];
+  const bool per = g.periodic != 0;
+  if (z0 > 1 && z1 < nz) return;
+  const uint32_t kb = it.kbase[lane % 9];
+  const bool there = seam == 0 ? per && z0 == 0 : seam == 1 ? z0 <= 1 : per && z1 == nz;
+  bool drop = false;
+  if (lane < 27 && there && (per || kb != kNoCell)) {
+    const uint32_t kl = kb + (uint32_t)max(z0 - 1, 0), kh = kb + (uint32_t)min(z1 + 1, nz);
+    // the cells before the seam and after it
+    const uint32_t a0 = seam == 0 ? kb + nz - 1 : kl, a1 = seam == 0 ? kb + nz : seam == 1 ? kb + 1 : kh;
+    const uint32_t c0 = seam == 0 ? kl : seam == 1 ? kb + 1 : kb, c1 = seam == 2 ? kb + 1 : kh;
+    const uint32_t sa = b.start[a0], ea = b.start[a1], sc = b.start[c0], ec = b.start[c1];
+    if (sa < ea && sc < ec) {
+      const float up = seam == 1 ? 0.0f : g.L[2];  // by an image below, or of one above
+      // (a NaN, last in cell 0, may hide atoms that are out of order before it)
+      drop = !(b.rs[ea - 1].z - (seam == 0 ? up : 0.0f) <= b.rs[sc].z + (seam == 2 ? up : 0.0f));
+    }
+  }
+  if (__any_sync(0xffffffffu, drop) && lane == 0) d.rcw = kFar;
+}
+
 // Moves the staged atoms into the item's frame, a warp per column (x - 0 is x,
 // so unshifted atoms pass unchanged).
 template <int NT, int kWarps>
@@ -539,7 +569,8 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
     l1b = d.lj4[tbt + 1];
   }
 
-  // the tile's z window (all z when its first atom is a far one)
+  // the tile's z window (all z when its first atom is a far one, or the columns are not
+  // sorted: check_order)
   const float z0 = E[hb].z, z1 = E[hb + min((uint32_t)kTile, H - h0) - 1].z;
   const float zlo = z0 < 1e29f ? z0 - d.rcw : -kFar, zhi = z1 + d.rcw;
   const uint32_t blocks = d.c0[9] >> 3;
@@ -793,6 +824,8 @@ __global__ void __launch_bounds__(kWarps * 32,
   if (warp == 0) {
     __syncwarp();
     plan_stage<NT>(b, it, d, E, &full);
+  } else if (warp == 2) {
+    check_order<NT>(b, it, d);
   }
   __syncthreads();
   if (!d.overflow) {

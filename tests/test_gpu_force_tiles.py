@@ -166,3 +166,27 @@ def test_pairs_that_do_not_interact(cuda_lib, ntypes, eps, acc64):
     got = p.get("F")[:, :3].astype(np.float64)
     assert np.sqrt(((got - F) ** 2).sum()) < BAR * scale
     assert p.status() == 0
+
+
+@pytest.mark.parametrize("up", [6.0, 60.0])
+@pytest.mark.parametrize("Lz", [14.0, 45.0])
+def test_open_box_atoms_above_the_top_face(cuda_lib, up, Lz):
+    """Atoms more than a cell above the top of an open box are filed in cell 0, among
+    atoms far below them: their column is not sorted by z.  One such atom or two above
+    every column (of one run and of two), at several alignments of the columns' blocks
+    and tiles."""
+    full = system((12.0, 11.0, Lz), 10 ** 6, 1, 11)
+    x, y = np.meshgrid(np.arange(1.25, 12, 2.5), np.arange(1.25, 12, 2.5), indexing="ij")
+    odd = (np.round(x / 2.5 - 0.5) + np.round(y / 2.5 - 0.5)) % 2 == 1
+    z = Lz + up + np.where(odd, 0.7, 0.0)
+    high = np.stack([x, y, z], -1).reshape(-1, 3)
+    high = np.concatenate([high, high[odd.reshape(-1)] + [0.0, 0.0, 1.1]])
+    rng = np.random.default_rng(3)
+    for k in range(16 if Lz < 20 else 6):
+        # any atoms but a few of the lowest cells, so that every column's cell 0 shifts
+        low = np.flatnonzero(full.r[:, 2] < 2.4)
+        keep = np.setdiff1d(np.arange(full.n), rng.permutation(low)[:5 * k])
+        r = np.concatenate([full.r[keep], high]).astype(np.float32).astype(np.float64)
+        s = W.LJSystem(box=full.box, r=r, v=np.zeros_like(r), mass=np.ones(len(r)),
+                       types=np.zeros(len(r), np.uint32), lj=full.lj, rc=2.5)
+        assert check(s, periodic=False) == 0
