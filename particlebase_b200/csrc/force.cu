@@ -44,7 +44,7 @@
 // operands, FP32 sums) gives 16 x 8 values
 // |x_j|^2 - 2 x_i . x_j + (|x_i|^2 - bound), whose sign says whether the pair
 // may be within rc.  `bound` exceeds rc^2 by what the rounding of the records
-// can change (from the largest norm staged), so the hits are a superset of the
+// can change (from the home atom's own norm), so the hits are a superset of the
 // pairs inside the cutoff: about 4 % more.  With several types the indicators'
 // share of the product lowers the bound to that pair of types' own cutoff.
 // mma.sync and not tcgen05: a tile shares its window with no other, its product
@@ -84,7 +84,7 @@ constexpr uint32_t kTabBytes = kTabBlocks * 4;
 __host__ __device__ constexpr uint32_t list_len(int nt) { return nt > 1 ? 36u : 28u; }
 // Per warp: the table of block starts, and the lanes' lists of hits.
 __host__ __device__ constexpr uint32_t warp_bytes(int nt) { return kTabBytes + list_len(nt) * 64u; }
-constexpr float kMaxNorm = 30000.f;  // largest norm the fp16 records are used for
+constexpr float kMaxNorm = 30000.f;  // largest norm of a home atom in fp16 records
 
 // One work item: its staged columns and the constants of its frame.
 template <int NT>
@@ -100,7 +100,7 @@ struct Stage {
   uint32_t kbase[9];
   int z0, nz, nseg, periodic, overflow;
   int shifted;            // some frame shift is not zero
-  uint32_t nmax;          // largest norm staged (float bits, non-negative)
+  uint32_t nmax;          // largest norm of a home atom (float bits, non-negative)
   LJLocal<NT> lj;
   // several types: what the bound of a pair of types lies below the longest
   // one, per type of home atom as fp16 for candidate types 0 .. 3
@@ -462,6 +462,7 @@ template <int NT, int kWarps>
 __device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf, uint32_t *Ht, float *zb) {
   const uint32_t total = d.c0[9];
   const float cx = d.cx, cy = d.cy, cz = d.cz, sc = d.scale;
+  const uint32_t hb = d.hb, H = d.H;
   float nmax = 0.f;
   for (uint32_t u = threadIdx.x; u < total + 8u; u += kWarps * 32) {
     const float4 q = E[u];
@@ -480,7 +481,7 @@ __device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf,
     }
     const float far = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
     if (far < 1e29f && !isnan(n))
-      nmax = fmaxf(nmax, n);
+      nmax = u - hb < H ? fmaxf(nmax, n) : nmax;
     else
       E[u] = make_float4(kFar, kFar, kFar, q.w);
     const uint32_t k = u & 7u;
@@ -533,13 +534,17 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
       a0 = t == 2 ? ca.x : ca.y;
       a1 = t == 2 ? cb.x : cb.y;
     }
-    // bound: rounding a record moves the point by at most 2^-11 of its norm,
-    // and the stored norm by 2^-11 of itself
-    const float nm = __uint_as_float(d.nmax), dl = sqrt_approx(nm) * (1.0f / 1024.0f);
-    const float bound =
-        d.rs2 + 1.05f * (2.0f * sqrt_approx(d.rs2) * dl + dl * dl + nm * (1.0f / 2048.0f)) + 1e-4f;
-    C[0] = C[1] = va ? fmaf(axy.x, axy.x, fmaf(axy.y, axy.y, az * az)) - bound : kFar;
-    C[2] = C[3] = vb ? fmaf(bxy.x, bxy.x, fmaf(bxy.y, bxy.y, bz * bz)) - bound : kFar;
+    // bound: rounding a record moves the point by at most 2^-11 of its distance from the
+    // centre, and the stored norm by 2^-11 of itself.  A partner within rc of a home atom
+    // lies at most rc farther from the centre, so each home atom has its own bound, which
+    // no atom far away widens.
+    const float rs = sqrt_approx(d.rs2) * 1.00001f;
+    const auto row = [&](float n) {
+      const float far = sqrt_approx(n) + rs, nm = far * far, dl = far * (1.0f / 1024.0f);
+      return n - (d.rs2 + 1.05f * (2.0f * rs * dl + dl * dl + nm * (1.0f / 2048.0f)) + 1e-4f);
+    };
+    C[0] = C[1] = va ? row(fmaf(axy.x, axy.x, fmaf(axy.y, axy.y, az * az))) : kFar;
+    C[2] = C[3] = vb ? row(fmaf(bxy.x, bxy.x, fmaf(bxy.y, bxy.y, bz * bz))) : kFar;
   }
   const uint32_t eb = smem_u32(E) + 32u * t;  // candidate 2 t of a block
   // B operand: candidate g; lanes t >= 2 hold its type indicators (one type:
@@ -848,7 +853,7 @@ __global__ void __launch_bounds__(kWarps * 32,
     make_records<NT, kWarps>(d, E, Hf, Ht, zb);
     __syncthreads();
   }
-  // records out of the fp16 range (atoms far outside their cells): global path
+  // home atoms out of the range of fp16 records (far outside their cells): global path
   const bool global = d.overflow || __uint_as_float(d.nmax) > kMaxNorm;
   const uint32_t ntile = d.ntile;
   for (uint32_t k = warp; k < ntile; k += kWarps) {

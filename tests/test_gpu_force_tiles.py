@@ -190,3 +190,20 @@ def test_open_box_atoms_above_the_top_face(cuda_lib, up, Lz):
         s = W.LJSystem(box=full.box, r=r, v=np.zeros_like(r), mass=np.ones(len(r)),
                        types=np.zeros(len(r), np.uint32), lj=full.lj, rc=2.5)
         assert check(s, periodic=False) == 0
+
+
+@pytest.mark.parametrize("ntypes", [1, 3])
+@pytest.mark.parametrize("far", [20.0, 150.0, 400.0, 430.0, 470.0, 640.0, 700.0, 5000.0])
+def test_open_box_pairs_far_outside(cuda_lib, far, ntypes):
+    """Bound pairs of atoms far from the box, beside which the box's own atoms keep their
+    forces: within the range of the fp16 records (some 173 cell edges for a home atom, 256
+    for a candidate's norm) and beyond it."""
+    s = system((12.0, 11.0, 14.0), 650, ntypes, 6)
+    y, z = np.arange(1.25, 11, 2.6), 1.25  # no two of them at the cutoff
+    first = np.concatenate([[(-far, a, z) for a in y], [(12.0 + far, a + 0.1, z + 5) for a in y],
+                            [(a, -far, z + 2.5) for a in y], [(a, 4.0, -far) for a in y]])
+    pairs = np.concatenate([first, first + [0.4, 0.7, 0.8]])
+    s.r = np.concatenate([s.r, pairs]).astype(np.float32).astype(np.float64)
+    s.v, s.mass = np.zeros_like(s.r), np.ones(len(s.r))
+    s.types = np.concatenate([s.types, np.arange(len(pairs)) % ntypes]).astype(np.uint32)
+    assert check(s, periodic=False) == 0
