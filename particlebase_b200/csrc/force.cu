@@ -95,7 +95,7 @@ struct Stage {
   float szl, szm, szh;    // frame shift of the low image, the middle run, the high image
   float cx, cy, cz, scale;  // centre and scale of the fp16 records
   float rcw;              // half-width of the z windows
-  float rs2;              // rc^2 (of the longest-ranged pair) in record units
+  float rs, rs2, rs_dl;   // rc (of the longest-ranged pair) in record units: for the bounds
   uint32_t home_g0, hb, H, ntile;  // home atoms: first sorted slot, first stage slot, count
   uint32_t kbase[9];
   int z0, nz, nseg, periodic, overflow;
@@ -277,7 +277,10 @@ __device__ __forceinline__ void load_lj(const ForceBufs &b, const SysDesc &S, St
     d.lj.sc_rc = b.sc_rc;
     d.lj.sc_f0 = b.sc_f0;
     d.rcw = sqrtf(rc2max) * 1.00001f + 1e-5f;
-    d.rs2 = rc2max * sc * sc;
+    const float rs = sqrtf(rc2max) * sc * 1.00001f;
+    d.rs = rs;
+    d.rs2 = rc2max * sc * sc + 1e-4f;
+    d.rs_dl = rs * (1.05f / 512.0f);
   }
 }
 
@@ -534,14 +537,13 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
       a0 = t == 2 ? ca.x : ca.y;
       a1 = t == 2 ? cb.x : cb.y;
     }
-    // bound: rounding a record moves the point by at most 2^-11 of its distance from the
-    // centre, and the stored norm by 2^-11 of itself.  A partner within rc of a home atom
-    // lies at most rc farther from the centre, so each home atom has its own bound, which
-    // no atom far away widens.
-    const float rs = sqrt_approx(d.rs2) * 1.00001f;
+    // bound of a home atom: a partner within rc lies at most rc farther from the centre, at
+    // `far`; rounding the two records moves the points by at most 2^-10 far, and the
+    // stored norm by 2^-11 far^2 (5 % more of both, and 1e-4 in rs2, for the sums' own
+    // rounding).  No atom farther away widens it.
     const auto row = [&](float n) {
-      const float far = sqrt_approx(n) + rs, nm = far * far, dl = far * (1.0f / 1024.0f);
-      return n - (d.rs2 + 1.05f * (2.0f * rs * dl + dl * dl + nm * (1.0f / 2048.0f)) + 1e-4f);
+      const float far = sqrt_approx(n) + d.rs;
+      return n - fmaf(far, fmaf(far, 1.05f * (1.0f / 2048.0f + 1.0f / 1048576.0f), d.rs_dl), d.rs2);
     };
     C[0] = C[1] = va ? row(fmaf(axy.x, axy.x, fmaf(axy.y, axy.y, az * az))) : kFar;
     C[2] = C[3] = vb ? row(fmaf(bxy.x, bxy.x, fmaf(bxy.y, bxy.y, bz * bz))) : kFar;
