@@ -126,6 +126,30 @@ __host__ __device__ __forceinline__ uint32_t smem_bytes(uint32_t cap, int warps,
   return padded_slots(cap) * slot_bytes(nt) + (uint32_t)warps * warp_bytes(nt);
 }
 
+// Coefficient of w^k in cos(pi sqrt(w) / 2).
+constexpr double cos_term(int k) {
+  double t = 1.0;
+  for (int j = 1; j <= k; ++j)
+    t *= -3.14159265358979323846 * 3.14159265358979323846 / 4 / (2 * j * (2 * j - 1));
+  return t;
+}
+
+template <int K = 0>
+__device__ __forceinline__ double cos_sum(double w) {
+  constexpr double t = cos_term(K);
+  if constexpr (K == 8)
+    return t;
+  else
+    return fma(cos_sum<K + 1>(w), w, t);
+}
+
+// f0 cos(pi r / 2 rc) / r of the soft-core force: the cosine's Taylor series in (r / rc)^2, in
+// FP64 (its terms up to the 8th leave 6e-13 inside the range), takes no root and no quotient.
+template <int M>
+__device__ __forceinline__ float soft_core(const LJLocal<M> &lj, float r2) {
+  return lj.sc_f0 * (float)cos_sum((double)r2 * lj.sc_w) * rsqrtf(r2);
+}
+
 // MODE kModeCapped: relaxation force of the steepest-descent path, with the
 // pair distance floored at sigma/2 so that overlapping random starts give
 // finite forces.  MODE kModeSoftCore: the soft-core force of potentialSC
@@ -139,10 +163,7 @@ struct PairAcc {
   __device__ __forceinline__ void add(const LJLocal<M> &lj, int k, float dx, float dy, float dz,
                                       float r2) {
     if (MODE == kModeSoftCore) {
-      const float r = sqrtf(r2);
-      if (r > lj.sc_rc) return;
-      const float mag = lj.sc_f0 * (float)cos((double)(r / lj.sc_rc) * 3.14159265358979323846 / 2);
-      const float f = mag * rsqrtf(r2);
+      const float f = soft_core(lj, r2);
       fx += (Acc)(f * dx);
       fy += (Acc)(f * dy);
       fz += (Acc)(f * dz);
@@ -274,8 +295,10 @@ __device__ __forceinline__ void load_lj(const ForceBufs &b, const SysDesc &S, St
     d.cut[lane] = make_uint2(pack_half2(c[0], c[1]), pack_half2(c[2], c[3]));
   }
   if (lane == 0) {
-    d.lj.sc_rc = b.sc_rc;
-    d.lj.sc_f0 = b.sc_f0;
+    if (MODE == kModeSoftCore) {
+      d.lj.sc_w = 1.0 / ((double)b.sc_rc * b.sc_rc);
+      d.lj.sc_f0 = b.sc_f0;
+    }
     d.rcw = sqrtf(rc2max) * 1.00001f + 1e-5f;
     const float rs = sqrtf(rc2max) * sc * 1.00001f;
     d.rs = rs;
@@ -501,7 +524,6 @@ template <int NT, bool ENERGY, typename Acc, int MODE>
 __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> &d,
                                             const float4 *E, const uint2 *Hf, const uint32_t *Ht,
                                             const float *zb, uint32_t tile, uint32_t *tab, double *ce) {
-  constexpr bool kPacked = MODE != kModeSoftCore;
   constexpr bool kSum32 = std::is_same<Acc, float>::value;
   const int lane = threadIdx.x & 31;
   const uint32_t g = (uint32_t)lane >> 2, t = (uint32_t)lane & 3u;
@@ -641,79 +663,78 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
           const float2 dz = make_float2(pa.z - q[j].z, pb.z - q[j].z);
           const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
           const int tj = NT == 1 ? 0 : __float_as_int(q[j].w);
-          if constexpr (kPacked) {
-            if (NT == 2) {
-              // both candidate types' parameters wait in registers
-              const bool k = tj != 0;
-              s2 = make_float2(k ? l1a.x : l0a.x, k ? l1b.x : l0b.x);
-              e24 = make_float2(k ? l1a.y : l0a.y, k ? l1b.y : l0b.y);
-              rca = __float_as_uint(k ? l1a.z : l0a.z);
-              rcb = __float_as_uint(k ? l1b.z : l0b.z);
-            } else if (NT > 2) {
-              const float4 la = d.lj4[ta + tj], lb = d.lj4[tbt + tj];
-              s2 = make_float2(la.x, lb.x);
-              e24 = make_float2(la.y, lb.y);
-              rca = __float_as_uint(la.z);
-              rcb = __float_as_uint(lb.z);
-            }
-            const bool ina = inside(r2.x, rca), inb = inside(r2.y, rcb);
-            float2 r2c = r2;
+          if (NT == 2) {
+            // both candidate types' parameters wait in registers
+            const bool k = tj != 0;
+            s2 = make_float2(k ? l1a.x : l0a.x, k ? l1b.x : l0b.x);
+            e24 = make_float2(k ? l1a.y : l0a.y, k ? l1b.y : l0b.y);
+            rca = __float_as_uint(k ? l1a.z : l0a.z);
+            rcb = __float_as_uint(k ? l1b.z : l0b.z);
+          } else if (NT > 2) {
+            const float4 la = d.lj4[ta + tj], lb = d.lj4[tbt + tj];
+            s2 = make_float2(la.x, lb.x);
+            e24 = make_float2(la.y, lb.y);
+            rca = __float_as_uint(la.z);
+            rcb = __float_as_uint(lb.z);
+          }
+          const bool ina = inside(r2.x, rca), inb = inside(r2.y, rcb);
+          float2 f, r2c = r2, sr6;
+          if constexpr (MODE == kModeSoftCore) {
+            f = sr6 = make_float2(0.0f, 0.0f);
+            if (ina || inb)  // (short ranges: seldom in any lane)
+              f = make_float2(soft_core(d.lj, r2.x), soft_core(d.lj, r2.y));
+          } else {
             if (MODE == kModeCapped) {
               const float2 fl = __fmul2_rn(make_float2(0.25f, 0.25f), s2);
               r2c = make_float2(fmaxf(r2.x, fl.x), fmaxf(r2.y, fl.y));
             }
             const float2 inv = make_float2(rcp_approx(r2c.x), rcp_approx(r2c.y));
             const float2 sr2 = __fmul2_rn(s2, inv);
-            const float2 sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
+            sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
             const float2 tt = __ffma2_rn(__fadd2_rn(e24, e24), sr6, make_float2(-e24.x, -e24.y));
-            float2 f = __fmul2_rn(__fmul2_rn(tt, sr6), inv);
-            f.x = ina ? f.x : 0.0f;
-            f.y = inb ? f.y : 0.0f;
-            if constexpr (kSum32) {
-              acc.fx = __ffma2_rn(f, dx, acc.fx);
-              acc.fy = __ffma2_rn(f, dy, acc.fy);
-              acc.fz = __ffma2_rn(f, dz, acc.fz);
-            } else {
-              const float2 gx = __fmul2_rn(f, dx), gy = __fmul2_rn(f, dy), gz = __fmul2_rn(f, dz);
-              acca.fx += (Acc)gx.x;
-              acca.fy += (Acc)gy.x;
-              acca.fz += (Acc)gz.x;
-              accb.fx += (Acc)gx.y;
-              accb.fy += (Acc)gy.y;
-              accb.fz += (Acc)gz.y;
-            }
-            if (ENERGY) {
-              const int ka = ta + tj, kb = tbt + tj;
-              if (NT > 1) e4 = make_float2(d.lj.e4[ka], d.lj.e4[kb]);
-              float2 u = __fmul2_rn(__fmul2_rn(e4, sr6), __fadd2_rn(sr6, m1));
-              u.x = ina ? u.x : 0.0f;
-              u.y = inb ? u.y : 0.0f;
-              // (a pair's half share is taken at the end: a power of two)
-              acca.pe += (Acc)u.x;
-              accb.pe += (Acc)u.y;
-              if (NT > 1) {  // one type: from pe and the count, at the end
-                acca.pes += (Acc)(ina ? u.x - d.lj.ush[ka] : 0.0f);
-                accb.pes += (Acc)(inb ? u.y - d.lj.ush[kb] : 0.0f);
-              }
-              // f is zero outside the cutoff, where r^2 may be +inf
-              acca.vir += (Acc)(ina ? f.x * r2c.x : 0.0f);
-              accb.vir += (Acc)(inb ? f.y * r2c.y : 0.0f);
-              acca.n += (uint32_t)ina + (uint32_t)inb;
-            }
+            f = __fmul2_rn(__fmul2_rn(tt, sr6), inv);
+          }
+          f.x = ina ? f.x : 0.0f;
+          f.y = inb ? f.y : 0.0f;
+          if constexpr (kSum32) {
+            acc.fx = __ffma2_rn(f, dx, acc.fx);
+            acc.fy = __ffma2_rn(f, dy, acc.fy);
+            acc.fz = __ffma2_rn(f, dz, acc.fz);
           } else {
-            if (r2.x < d.lj.rc2[ta + tj] && r2.x > 0.0f)
-              acca.add(d.lj, ta + tj, dx.x, dy.x, dz.x, r2.x);
-            if (r2.y < d.lj.rc2[tbt + tj] && r2.y > 0.0f)
-              accb.add(d.lj, tbt + tj, dx.y, dy.y, dz.y, r2.y);
+            const float2 gx = __fmul2_rn(f, dx), gy = __fmul2_rn(f, dy), gz = __fmul2_rn(f, dz);
+            acca.fx += (Acc)gx.x;
+            acca.fy += (Acc)gy.x;
+            acca.fz += (Acc)gz.x;
+            accb.fx += (Acc)gx.y;
+            accb.fy += (Acc)gy.y;
+            accb.fz += (Acc)gz.y;
+          }
+          if (ENERGY) {
+            const int ka = ta + tj, kb = tbt + tj;
+            if (NT > 1) e4 = make_float2(d.lj.e4[ka], d.lj.e4[kb]);
+            float2 u = __fmul2_rn(__fmul2_rn(e4, sr6), __fadd2_rn(sr6, m1));
+            u.x = ina ? u.x : 0.0f;
+            u.y = inb ? u.y : 0.0f;
+            // (a pair's half share is taken at the end: a power of two)
+            acca.pe += (Acc)u.x;
+            accb.pe += (Acc)u.y;
+            if (NT > 1) {  // one type: from pe and the count, at the end
+              acca.pes += (Acc)(ina ? u.x - d.lj.ush[ka] : 0.0f);
+              accb.pes += (Acc)(inb ? u.y - d.lj.ush[kb] : 0.0f);
+            }
+            // f is zero outside the cutoff, where r^2 may be +inf
+            acca.vir += (Acc)(ina ? f.x * r2c.x : 0.0f);
+            accb.vir += (Acc)(inb ? f.y * r2c.y : 0.0f);
+            acca.n += (uint32_t)ina + (uint32_t)inb;
           }
         }
       }
     } while (u < cb4);
   }
   // the 4 lanes of an atom
-  using Sum = typename std::conditional<kPacked && kSum32, float, Acc>::type;
+  using Sum = typename std::conditional<kSum32, float, Acc>::type;
   Sum v[6] = {(Sum)acca.fx, (Sum)acca.fy, (Sum)acca.fz, (Sum)accb.fx, (Sum)accb.fy, (Sum)accb.fz};
-  if constexpr (kPacked && kSum32) {
+  if constexpr (kSum32) {
     v[0] = acc.fx.x;
     v[1] = acc.fy.x;
     v[2] = acc.fz.x;
@@ -731,10 +752,8 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
   if (ENERGY) {
     double e[4] = {warp_sum((double)(acca.pe + accb.pe)), warp_sum((double)(acca.pes + accb.pes)),
                    warp_sum((double)(acca.vir + accb.vir)), (double)warp_sum(acca.n + accb.n)};
-    if (kPacked) {
-      if (NT == 1) e[1] = e[0] - e[3] * (double)d.lj.ush[0];
-      for (int k = 0; k < 3; ++k) e[k] *= 0.5;
-    }
+    if (NT == 1) e[1] = e[0] - e[3] * (double)d.lj.ush[0];
+    for (int k = 0; k < 3; ++k) e[k] *= 0.5;
     if (lane == 0)
       for (int k = 0; k < 4; ++k) ce[k] = e[k];
   }

@@ -26,7 +26,8 @@ static_assert(kChunk == 16, "the quad table layout holds chunks of 16 quads");
 template <int NT>
 struct LJLocal {
   float s2[NT * NT], e24[NT * NT], e4[NT * NT], rc2[NT * NT], ush[NT * NT];
-  float sc_rc, sc_f0;  // soft-core mode: range and strength
+  double sc_w;  // soft-core mode: 1 / range^2
+  float sc_f0;  // and strength
 };
 
 // Pair force laws of the kernel.

@@ -207,3 +207,33 @@ def test_open_box_pairs_far_outside(cuda_lib, far, ntypes):
     s.v, s.mass = np.zeros_like(s.r), np.ones(len(s.r))
     s.types = np.concatenate([s.types, np.arange(len(pairs)) % ntypes]).astype(np.uint32)
     assert check(s, periodic=False) == 0
+
+
+@pytest.mark.parametrize("ntypes", [1, 2, 5])
+@pytest.mark.parametrize("rc", [0.9, 2.0, 2.5, 3.1])
+def test_soft_core(cuda_lib, ntypes, rc):
+    """f0 cos(pi r / 2 rc) along r, within rc and the pair's own cutoff, against all pairs in
+    FP64; also where the range ends beyond the cutoff, and in cells that go to global memory
+    (a dense ball)."""
+    from particlebase_b200.md import from_system
+    a = system((9.0, 10.5, 16.0), 900, ntypes, 30 + ntypes)
+    b = system((20.0, 20.0, 20.0), 600, ntypes, 5)
+    ball = 10.0 + np.random.default_rng(1).uniform(-1.5, 1.5, (2500, 3))
+    b.r = np.concatenate([b.r, ball]).astype(np.float32).astype(np.float64)
+    b.v, b.mass = np.zeros_like(b.r), np.ones(len(b.r))
+    b.types = (np.arange(len(b.r)) % ntypes).astype(np.uint32)
+    for s, overflow in ((a, 0), (b, 1)):
+        d = s.r[:, None] - s.r[None]
+        d -= s.L * np.round(d / s.L)
+        r2 = (d ** 2).sum(-1)
+        pair = s.lj[s.types[:, None], s.types[None], 2]
+        r = np.sqrt(r2)
+        near = (r < np.minimum(rc, pair)) & (r2 > 0)
+        f = np.where(near, 10.0 * np.cos(np.pi / 2 * r / rc) / np.where(near, r, 1.0), 0.0)
+        F = (f[..., None] * d).sum(1)
+        p = from_system(s)
+        p.calcBlockID()
+        p.calcForceSoftCore(rc, 10.0)
+        got = p.get("F")[:, :3].astype(np.float64)
+        assert np.sqrt(((got - F) ** 2).sum()) < BAR * np.sqrt((F ** 2).sum())
+        assert p.status() == overflow
