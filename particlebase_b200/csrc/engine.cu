@@ -717,8 +717,10 @@ int engine_setup_cells(Engine &e) {
     const double apc = (double)P.n / g.ncells;
     apc_max = std::max(apc_max, apc);
     const bool half = (e.flags & PB_MD_HALF_SHELL) && !(e.flags & PB_MD_ACC_FP64);
-    P.seg = choose_segment(apc, g.n[2], e.seg_scale, P.lj_set ? P.lj.nt : 1, half);
-    P.cap = (uint32_t)choose_capacity(apc, P.seg);
+    const int nt = P.lj_set ? P.lj.nt : 1;
+    P.seg = choose_segment(apc, g.n[2], e.seg_scale, nt, half);
+    // (CTAs of 128 threads: more of them fit as they are)
+    P.cap = (uint32_t)choose_capacity(apc, P.seg, nt, e.force_threads != 128);
     P.cap_half = (uint32_t)choose_capacity_half(apc, P.seg);
     e.cap_max = std::max(e.cap_max, P.cap);
     e.cap_half_max = std::max(e.cap_half_max, P.cap_half);

@@ -519,7 +519,7 @@ __device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf,
 }
 
 // One tile of 16 home atoms (one warp); energy sums (pe, shifted pe, virial,
-// pairs) in `ce`.
+// pairs) are added to `ce`.
 template <int NT, bool ENERGY, typename Acc, int MODE>
 __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> &d,
                                             const float4 *E, const uint2 *Hf, const uint32_t *Ht,
@@ -755,7 +755,7 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
     if (NT == 1) e[1] = e[0] - e[3] * (double)d.lj.ush[0];
     for (int k = 0; k < 3; ++k) e[k] *= 0.5;
     if (lane == 0)
-      for (int k = 0; k < 4; ++k) ce[k] = e[k];
+      for (int k = 0; k < 4; ++k) ce[k] += e[k];
   }
 }
 
@@ -809,7 +809,7 @@ __device__ __noinline__ void task_global(const ForceBufs &b, const Stage<NT> &d,
     }
   }
   if (ENERGY && lane == 0)
-    for (int k = 0; k < 4; ++k) ce[k] = s[k];
+    for (int k = 0; k < 4; ++k) ce[k] += s[k];
 }
 
 // ---- the kernel ---------------------------------------------------------------
@@ -821,7 +821,7 @@ __global__ void __launch_bounds__(kWarps * 32,
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ Stage<NT> d;
   __shared__ uint64_t full;
-  __shared__ double cle[ENERGY ? kWinCap : 1][4];
+  __shared__ double cle[ENERGY ? kWarps : 1][4];  // energy sums of the warps
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const ForceItem &it = b.items[blockIdx.x];
   const uint32_t sys = it.sys;
@@ -877,18 +877,20 @@ __global__ void __launch_bounds__(kWarps * 32,
   // home atoms out of the range of fp16 records (far outside their cells): global path
   const bool global = d.overflow || __uint_as_float(d.nmax) > kMaxNorm;
   const uint32_t ntile = d.ntile;
+  double *ce = cle[ENERGY ? warp : 0];
+  if (ENERGY && lane == 0)
+    for (int k = 0; k < 4; ++k) ce[k] = 0.0;
   for (uint32_t k = warp; k < ntile; k += kWarps) {
-    double *ce = cle[ENERGY ? k : 0];
     if (!global)
       tile_forces<NT, ENERGY, Acc, MODE>(b, d, E, Hf, Ht, zb, k, tab, ce);
     else
       task_global<NT, ENERGY, Acc, MODE>(b, d, k, ntile, ce);
   }
-  if (ENERGY) {  // the item's sums in tile order
+  if (ENERGY) {  // the item's sums in the order of its warps
     __syncthreads();
     if (threadIdx.x < 4) {
       double v = 0.0;
-      for (uint32_t k = 0; k < ntile; ++k) v += cle[k][threadIdx.x];
+      for (int k = 0; k < kWarps; ++k) v += cle[k][threadIdx.x];
       b.partials[(size_t)blockIdx.x * 4 + threadIdx.x] = v;
     }
   }
@@ -944,17 +946,35 @@ int force_max_capacity() {
   return (int)cap;
 }
 
-int force_smem_per_cta(int cap, int nt) {
-  // dynamic part, and a bound of the static part (stage record, energy sums)
+// Static shared memory of a CTA, at most: the stage record, and the energy sums.
+static int static_bytes(int nt, bool energy) {
   const size_t st = nt <= 1 ? sizeof(Stage<1>) : nt <= 2 ? sizeof(Stage<2>)
                     : nt <= 4 ? sizeof(Stage<4>) : sizeof(Stage<8>);
-  return (int)(smem_bytes((uint32_t)cap, kWarpsDefault, nt) + st + kWinCap * 4 * 8 + 64);
+  return (int)st + (energy ? kWarpsDefault : 1) * 4 * 8 + 64;
+}
+
+int force_smem_per_cta(int cap, int nt) {
+  // (1.5 KB over the stage record: runs that would fill the last of it leave a stage no
+  // headroom)
+  return (int)smem_bytes((uint32_t)cap, kWarpsDefault, nt) + static_bytes(nt, false) + 1536;
 }
 
 int force_smem_limit(int nt) {
   // the CTAs per SM that the registers allow (one type 4, several 3) share its
   // 228 KB, less 1 KB per CTA reserved by the driver
   return (nt <= 1 ? 56 : 74) * 1024;
+}
+
+int force_capacity_room(int nt) {
+  // With one type the launches with energies have fewer CTAs per SM by their registers and
+  // more shared memory each; and a one-type system may run beside systems of many types,
+  // whose slots are larger.
+  const auto fits = [](uint32_t cap, int k, bool energy) {
+    return (int)smem_bytes(cap, kWarpsDefault, k) + static_bytes(k, energy) <= force_smem_limit(k);
+  };
+  uint32_t cap = 64;
+  while (fits(cap + 16, nt, nt > 1) && (nt > 1 || fits(cap + 16, kMaxTypes, false))) cap += 16;
+  return (int)cap;
 }
 
 cudaError_t launch_force_capped(const ForceBufs &b, int nt_max, cudaStream_t s) {

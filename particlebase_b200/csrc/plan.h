@@ -35,8 +35,9 @@ int choose_segment(double atoms_per_cell, int nz, double scale = 1.0, int nt = 1
                    bool half = false);
 
 // Shared-memory capacity (atoms) of a force CTA staging 9 columns x (seg + 2)
-// cells at the given mean occupancy, with headroom for fluctuations.
-int choose_capacity(double atoms_per_cell, int seg);
+// cells at the given mean occupancy of a system of `nt` types, with headroom for
+// fluctuations; `spare`: and whatever else the CTAs of an SM have room for.
+int choose_capacity(double atoms_per_cell, int seg, int nt, bool spare);
 // Member slots per cell bucket of the two-kernel cell build: at least 32 and
 // about twice the mean occupancy (a fuller cell spills to the overflow list).
 int choose_bucket_cap(double atoms_per_cell);
@@ -55,8 +56,11 @@ void append_items(uint32_t sys, const Grid &g, int seg, uint32_t cell0,
 int force_max_segment();
 // Largest staged-atom capacity of a force CTA.
 int force_max_capacity();
-// Shared memory (dynamic plus an upper bound of the static part) of one
-// default-shape force CTA with staged-atom capacity `cap` and `nt` types.
+// The largest capacity with which the CTAs per SM that the default launch shape is built
+// for stay resident.
+int force_capacity_room(int nt);
+// Shared memory of one default-shape force CTA with staged-atom capacity `cap` and
+// `nt` types, with a margin.
 int force_smem_per_cta(int cap, int nt);
 // The shared memory a default-shape force CTA may use so that the CTAs per SM
 // its launch shape is built for stay resident.

@@ -237,3 +237,31 @@ def test_soft_core(cuda_lib, ntypes, rc):
         got = p.get("F")[:, :3].astype(np.float64)
         assert np.sqrt(((got - F) ** 2).sum()) < BAR * np.sqrt((F ** 2).sum())
         assert p.status() == overflow
+
+
+@pytest.mark.parametrize("ntypes,fill", [(1, 0.78), (1, 0.8), (2, 0.76), (2, 0.8)])
+def test_density_contrast_that_fits_the_stage(cuda_lib, po, ntypes, fill):
+    """A slab of liquid with empty space above it: the items inside it hold up to 1 / fill
+    times the mean occupancy, which the stage has room for; an item that does not fit takes
+    the slower global path and raises the status word."""
+    from particlebase_b200.md import from_system
+    L = np.array([20.0, 20.0, 150.0])
+    k = np.round(L / (4 / 0.8442) ** (1 / 3)).astype(int)
+    g = np.stack(np.meshgrid(*[np.arange(x) for x in k], indexing="ij"), -1).reshape(-1, 1, 3)
+    r = (g + np.array([[0, 0, 0], [.5, .5, 0], [.5, 0, .5], [0, .5, .5]]) + 0.25).reshape(-1, 3) / k * L
+    r = r[r[:, 2] < fill * L[2]]
+    r += np.random.default_rng(2).normal(0, 0.05, r.shape)
+    r = r.astype(np.float32).astype(np.float64)
+    lj = np.ones((ntypes, ntypes, 3)) * [1.0, 1.0, 2.5]
+    s = W.LJSystem(box=np.array([0, L[0], 0, L[1], 0, L[2]], np.float32), r=r, v=np.zeros_like(r),
+                   mass=np.ones(len(r)), types=(np.arange(len(r)) % ntypes).astype(np.uint32),
+                   lj=lj, rc=2.5)
+    p = from_system(s)
+    p.calcBlockID()
+    p.calcForce()
+    assert p.status() == 0
+    O = po.Oracle(s.box, s.lj, s.rc, s.r, types=s.types)
+    O.forces()
+    F = O.get("F")
+    got = p.get("F")[:, :3].astype(np.float64)
+    assert np.sqrt(((got - F) ** 2).sum()) < BAR * np.sqrt((F ** 2).sum())
