@@ -100,6 +100,7 @@ struct Stage {
   uint32_t kbase[9];
   int z0, nz, nseg, periodic, overflow;
   int shifted;            // some frame shift is not zero
+  int one;                // the system has one type, whatever the launch is compiled for
   uint32_t nmax;          // largest norm of a home atom (float bits, non-negative)
   LJLocal<NT> lj;
   // several types: what the bound of a pair of types lies below the longest
@@ -299,6 +300,7 @@ __device__ __forceinline__ void load_lj(const ForceBufs &b, const SysDesc &S, St
       d.lj.sc_w = 1.0 / ((double)b.sc_rc * b.sc_rc);
       d.lj.sc_f0 = b.sc_f0;
     }
+    d.one = T.nt == 1;
     d.rcw = sqrtf(rc2max) * 1.00001f + 1e-5f;
     const float rs = sqrtf(rc2max) * sc * 1.00001f;
     d.rs = rs;
@@ -752,7 +754,8 @@ __device__ __forceinline__ void tile_forces(const ForceBufs &b, const Stage<NT> 
   if (ENERGY) {
     double e[4] = {warp_sum((double)(acca.pe + accb.pe)), warp_sum((double)(acca.pes + accb.pes)),
                    warp_sum((double)(acca.vir + accb.vir)), (double)warp_sum(acca.n + accb.n)};
-    if (NT == 1) e[1] = e[0] - e[3] * (double)d.lj.ush[0];
+    // (the same sum when the system runs beside others of more types)
+    if (NT == 1 || d.one) e[1] = e[0] - e[3] * (double)d.lj.ush[0];
     for (int k = 0; k < 3; ++k) e[k] *= 0.5;
     if (lane == 0)
       for (int k = 0; k < 4; ++k) ce[k] += e[k];

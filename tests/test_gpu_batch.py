@@ -90,6 +90,27 @@ def test_batch_forces_vs_oracle(cuda_lib, po):
         assert abs(sums[k, 2] - info["pe"]) <= 1e-5 * abs(info["pe"]) + 1e-6, f"pe {k}"
 
 
+@pytest.mark.parametrize("fp64_forces", [False, True])
+def test_energies_equal_alone_beside_systems_of_more_types(cuda_lib, fp64_forces):
+    """The largest number of types in a batch picks the force kernel of all its systems;
+    a system's energies, shifted energy included, have the same bits as alone."""
+    from particlebase_b200.batch import Batch
+    systems = perturbed(replicas(2, seed=21))
+    systems.append(W.kob_andersen_random(3000, 1.2, 0.8, seed=6))  # two types
+    three = W.kob_andersen_random(2000, 1.2, 0.8, seed=7)
+    lj = np.ones((3, 3, 3)) * [1.0, 1.0, 2.5]
+    lj[:2, :2] = three.lj
+    three.lj, three.types = lj, three.types + (np.arange(three.n) % 5 == 0).astype(np.uint32)
+    for group in (systems, systems + [three]):
+        b = Batch.from_systems(group, dt=DT, fp64_forces=fp64_forces)
+        b.force(energy=True)
+        got = b.sums()
+        for k, s in enumerate(group):
+            a = Batch.from_systems([s], dt=DT, fp64_forces=fp64_forces)
+            a.force(energy=True)
+            assert_same(got[k], a.sums()[0], f"sums of system {k}")
+
+
 def test_repack_continues_bitwise(cuda_lib):
     """Systems that stay through a repack, and systems admitted by it, follow
     the same trajectory as when run alone from the start."""
