@@ -161,8 +161,10 @@ int pb_md_force(pb_md *h, uint32_t flags);
  * withhold their first buffer), with every wait for it bounded by `polls` polls
  * of at most 1 us.  The wait runs out, the CTAs end early, the call returns
  * PB_OK and the status word carries PB_STATUS_WAIT_TIMEOUT; the forces of that
- * call are not meaningful.  The
+ * call are not meaningful.  With PB_WAIT_TEST_ENERGY added to `polls` the call
+ * has PB_FORCE_ENERGY, and its sums hold nothing of the items that timed out.  The
  * handle stays usable: the next pb_md_force is complete again. */
+#define PB_WAIT_TEST_ENERGY 0x80000000u
 int pb_md_force_wait_test(pb_md *h, uint32_t polls);
 /* cudaParticleVV::clearForce (cudaParticleVV.cu:10-15): F = Fold = 0. */
 int pb_md_clear_force(pb_md *h);

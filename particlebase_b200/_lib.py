@@ -26,6 +26,7 @@ FIELD = {
 VEL_FP64 = 0x1
 ACC_FP64 = 0x2
 HALF_SHELL = 0x4
+WAIT_TEST_ENERGY = 0x80000000
 FORCE_ENERGY = 0x1
 MODE_VV = 0
 MODE_GAUSS = 1

@@ -868,6 +868,8 @@ __global__ void __launch_bounds__(kWarps * 32,
         atomicOr(&b.status[sys], kStatusWaitTimeout);
         if (!(b.test_flags & 1u)) mbar_wait_bounded(&full, 0u);
       }
+      // not what an earlier call left there
+      if (ENERGY && threadIdx.x < 4) b.partials[(size_t)blockIdx.x * 4 + threadIdx.x] = 0.0;
       return;
     }
     if (d.shifted) {

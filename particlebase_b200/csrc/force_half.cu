@@ -821,7 +821,10 @@ __global__ void __launch_bounds__((kProd + kCons) * 32, 2) k_force_half(ForceBuf
       if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(b.queue + 1, 1u) == gridDim.x - 1) {
-          atomicExch(b.queue, 0u);
+          const uint32_t claimed = atomicExch(b.queue, 0u);
+          // items that no CTA took before all gave up
+          if (ENERGY)
+            for (size_t k = (size_t)claimed * 4; k < (size_t)b.nitems * 4; ++k) b.partials[k] = 0.0;
           atomicExch(b.queue + 1, 0u);
         }
       }
@@ -849,6 +852,9 @@ __global__ void __launch_bounds__((kProd + kCons) * 32, 2) k_force_half(ForceBuf
         }
         break;
       }
+      // until the item is retired, not what an earlier call left there
+      if (ENERGY && threadIdx.x == 0)
+        for (int c = 0; c < 4; ++c) b.partials[(size_t)item * 4 + c] = 0.0;
       const bool ok = produce_item3<NT, kProd>(b, item, desc[bf], sc, stage(bf), &landed[bf],
                                                bf ? lphase1 : lphase0, running, kCons);
       if (!ok) {

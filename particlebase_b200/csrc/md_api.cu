@@ -208,10 +208,12 @@ int pb_md_force(pb_md *h, uint32_t flags) {
 }
 
 int pb_md_force_wait_test(pb_md *h, uint32_t polls) {
+  const bool energy = (polls & PB_WAIT_TEST_ENERGY) != 0;
+  polls &= ~PB_WAIT_TEST_ENERGY;
   if (!h || polls == 0) return PB_ERR_ARG;
   h->e.force_test_flags = 1u;
   h->e.force_wait_polls = polls;
-  const int rc = engine_force(h->e, false);
+  const int rc = engine_force(h->e, energy);
   h->e.force_test_flags = 0u;
   h->e.force_wait_polls = 0u;
   if (rc) return rc;

@@ -178,11 +178,12 @@ class MDSystem:
                                    out.ctypes.data_as(C.c_void_p), C.byref(n)), "gr")
         return out
 
-    def force_wait_test(self, polls: int = 2000) -> None:
+    def force_wait_test(self, polls: int = 2000, energy: bool = False) -> None:
         """Failure-detection test hook: one force call whose hand-off wait is
         made to run out (pb_md_force_wait_test); raises nothing, sets
         PB_STATUS_WAIT_TIMEOUT in the status word."""
-        self._ck(self.lib.pb_md_force_wait_test(self.h, int(polls)), "force_wait_test")
+        self._ck(self.lib.pb_md_force_wait_test(
+            self.h, int(polls) | (L.WAIT_TEST_ENERGY if energy else 0)), "force_wait_test")
 
     def clearForce(self) -> None:
         self._ck(self.lib.pb_md_clear_force(self.h), "clear_force")

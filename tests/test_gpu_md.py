@@ -565,3 +565,23 @@ def test_type_ids_beyond_the_tables(cuda_lib, half):
     again.set(0, "type", two.types)
     again.force()
     assert np.array_equal(again.get(1, "F"), F)
+
+
+@pytest.mark.parametrize("half", [False, True])
+def test_energies_of_a_force_call_that_timed_out_are_not_an_earlier_call_s(cuda_lib, half):
+    """The items whose wait ran out report no energy: the sums are not those of the
+    last complete call."""
+    s = perturbed(W.config_c1(), 0.05, 3)
+    p = md(cuda_lib, s, half_shell=half)
+    p.calcBlockID()
+    p.calcForce(energy=True)
+    before = p.sums()
+    assert before["pe"] < 0
+    p.force_wait_test(2000, energy=True)
+    assert p.status() & 0x4, "PB_STATUS_WAIT_TIMEOUT"
+    after = p.sums()
+    assert after["pe"] == after["pe_shift"] == after["virial"] == 0
+    p.calcForce(energy=True)
+    assert p.status() == 0
+    again = p.sums()
+    assert all(again[k] == before[k] for k in ("pe", "pe_shift", "virial"))
