@@ -111,3 +111,29 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(L, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(ImportError):
         L.lib()
+
+
+@pytest.mark.parametrize("flags,per_atom", [
+    # r, both forces, sorted positions; minv, mass, key, ticket, member and particle ids;
+    # overflow list; type; velocities
+    (0, 4 * 16 + 6 * 4 + 8 + 2 + 16),
+    (L.VEL_FP64, 4 * 16 + 6 * 4 + 8 + 2 + 24),
+    # the half shell's mirrors and fixed-point sums, which FP64 sums do without
+    (L.HALF_SHELL, 4 * 16 + 6 * 4 + 8 + 2 + 16 + 16 + 48),
+    (L.HALF_SHELL | L.ACC_FP64, 4 * 16 + 6 * 4 + 8 + 2 + 16),
+])
+def test_memory_estimate_counts_the_arrays_an_engine_has(lib, flags, per_atom):
+    """One atom more in the same cells and blocks costs what the engine's arrays hold per
+    atom; beside a second system also its system index."""
+    cell = np.tile(np.array([0, 50, 0, 50, 0, 50], np.float32), 2)
+    rc = np.full(2, 2.5, np.float32)
+
+    def total(*natoms):
+        n = np.array(natoms, np.uint32)
+        out = C.c_size_t()
+        assert lib.pb_batch_estimate_bytes(n.ctypes.data, cell.ctypes.data, rc.ctypes.data,
+                                           len(n), flags, C.byref(out)) == 0
+        return out.value
+
+    assert total(5002) - total(5001) == per_atom
+    assert total(5002, 700) - total(5001, 700) == per_atom + 4
