@@ -291,7 +291,9 @@ int pb_md_pair_stats(pb_md *h, double out[2]) {
     const double nc = start[k + 1] - start[k];
     double around = 0;
     for (int j = 0; j < 27; ++j) {
-      const uint32_t kn = P.key_of_ref[nb[(size_t)ref * 27 + j]];
+      const uint32_t r = nb[(size_t)ref * 27 + j];
+      if (r == kNoCell) continue;  // past a face of an open box
+      const uint32_t kn = P.key_of_ref[r];
       around += start[kn + 1] - start[kn];
     }
     cand += nc * (around - 1.0);

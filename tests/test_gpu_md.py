@@ -585,3 +585,18 @@ def test_energies_of_a_force_call_that_timed_out_are_not_an_earlier_call_s(cuda_
     assert p.status() == 0
     again = p.sums()
     assert all(again[k] == before[k] for k in ("pe", "pe_shift", "virial"))
+
+
+def test_pair_stats_of_an_open_box(cuda_lib, golden):
+    """Candidates of an open box: no neighbour cell past a face."""
+    r = golden["open_r4"][:, :3].astype(np.float64)
+    s = W.LJSystem(box=np.array([0, 20, 0, 20, 0, 20], np.float32), r=r, v=np.zeros_like(r),
+                   mass=np.ones(len(r)), types=np.zeros(len(r), np.uint32),
+                   lj=W.single_type_lj(), rc=2.5)
+    p = md(cuda_lib, s)
+    p.setupCutoffBlock(2.5, periodic=False)
+    p.calcBlockID()
+    cells = np.bincount(golden["open_cell_of"], minlength=len(golden["open_neighbors"]))
+    around = np.append(cells, 0)[np.minimum(golden["open_neighbors"], len(cells))].sum(1)
+    assert p.pair_stats()["ncand"] == (cells * (around - 1.0)).sum()
+    p.close()
