@@ -941,7 +941,7 @@ int engine_build(Engine &e) {
   return PB_OK;
 }
 
-// The force kernels take cell starts and sorted positions as they find them:
+// Force kernels and getters take cell starts and sorted positions as they find them:
 // before the first build these arrays hold whatever the pool last kept there.
 int engine_need_cells(Engine &e) { return e.cells_built ? PB_OK : engine_build(e); }
 

@@ -139,6 +139,7 @@ int engine_setup_cells(Engine &e);
 bool engine_ready(const Engine &e);
 
 int engine_build(Engine &e);
+int engine_need_cells(Engine &e);  // builds them if no build has been issued since the set-up
 int engine_force(Engine &e, bool energy);
 // Notes the type ids a caller writes for a system (uint16 per atom).
 void engine_note_types(Engine &e, uint32_t sys, const void *ids);

@@ -277,6 +277,7 @@ int pb_md_pair_stats(pb_md *h, double out[2]) {
   Engine &e = h->e;
   const SysParams &P = h->p();
   const uint32_t C = P.grid.ncells;
+  if (const int err = engine_need_cells(e)) return err;
   std::vector<uint32_t> start(C + 1);
   H_CUDA(cudaMemcpyAsync(start.data(), e.start, 4 * (size_t)(C + 1), cudaMemcpyDeviceToHost,
                          e.stream));
@@ -396,6 +397,8 @@ int pb_md_get(pb_md *h, int field, void *host, size_t bytes) {
   const bool cell_field = field >= PB_FIELD_CELL_OF && field <= PB_FIELD_R_SORTED;
   if (cell_field && !e.cells_ready) return fail(h, PB_ERR_STATE, "no cell list");
   if (bytes != need) return fail(h, PB_ERR_ARG, "size mismatch for field");
+  if (cell_field && field != PB_FIELD_CELL_KEY && field != PB_FIELD_NEIGHBORS)
+    if (const int err = engine_need_cells(e)) return err;
   const void *src = nullptr;
   switch (field) {
     case PB_FIELD_R: src = e.r; break;

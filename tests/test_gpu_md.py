@@ -600,3 +600,17 @@ def test_pair_stats_of_an_open_box(cuda_lib, golden):
     around = np.append(cells, 0)[np.minimum(golden["open_neighbors"], len(cells))].sum(1)
     assert p.pair_stats()["ncand"] == (cells * (around - 1.0)).sum()
     p.close()
+
+
+def test_cell_fields_without_a_cell_build(cuda_lib):
+    """Reading the cell list before the first build builds it."""
+    s = perturbed(W.config_c1(), 0.05, 3)
+    p = md(cuda_lib, s)
+    p.calcBlockID()
+    want = {f: p.get(f) for f in ("cell_of", "pid", "cell_start", "r_sorted")}
+    ncand = p.pair_stats()["ncand"]
+    for f, w in want.items():
+        q = md(cuda_lib, s)
+        assert np.array_equal(q.get(f), w), f
+        q.close()
+    assert md(cuda_lib, s).pair_stats()["ncand"] == ncand
