@@ -179,19 +179,7 @@ __device__ __forceinline__ void write_mirror_of(const CellBufs &b, const SysDesc
 
 __device__ __forceinline__ void write_mirror(const CellBufs &b, uint32_t me, uint32_t s,
                                              const float4 &p, uint32_t key) {
-  const SysDesc &S = b.sys[system_of(b, me)];
-  const uint32_t m = S.mirror0 + (s - S.atom0);
-  float x = p.x, y = p.y, z = p.z;
-  if (!isfinite(x) || !isfinite(y) || !isfinite(z)) {
-    const uint32_t d2 = (key - S.cell0) % (uint32_t)S.g.n[2];
-    x = 1e30f;
-    y = 1e30f;
-    z = S.g.lo[2] + (float)(d2 + 1) * S.g.len[2];
-  }
-  b.xs[m] = x;
-  b.ys[m] = y;
-  b.zs[m] = z;
-  b.ts[m] = (uint32_t)b.type[me];
+  write_mirror_of(b, b.sys[system_of(b, me)], s, p, key, (uint32_t)b.type[me]);
 }
 
 // Order key of a z coordinate: monotone in z for all non-NaN values (-0 and
@@ -514,7 +502,7 @@ __global__ void __launch_bounds__(kT, kMin) k_canon_tiles(CellBufs b) {
       }
     }
   } else {
-    // one warp per two cells, 16 cells per round
+    // one warp per two cells
     for (uint32_t r = 0; r < (1u << kTileShift); r += 2 * (kT / 32)) {
       const uint32_t k0 = r + 2 * (uint32_t)warp;
       const uint32_t ca = c0 + k0;

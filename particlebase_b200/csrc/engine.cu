@@ -802,12 +802,11 @@ int engine_setup_cells(Engine &e) {
             dalloc(e, &e.colxy, ncols) == cudaSuccess &&
             dalloc(e, &e.d_sys, e.nsys) == cudaSuccess && dalloc(e, &e.d_items, nitems) == cudaSuccess &&
             dalloc(e, &e.d_item0, e.nsys + 1) == cudaSuccess &&
-            dalloc(e, &e.fpartials, (size_t)4 * nitems) == cudaSuccess &&
-            dalloc(e, &e.fqueue, 2) == cudaSuccess;
-  // the half-shell kernel stages from structure-of-arrays mirrors; nobody else
-  // reads them, so the cell build writes them only where that kernel runs
+            dalloc(e, &e.fpartials, (size_t)4 * nitems) == cudaSuccess;
+  // the half-shell kernel claims items from a queue and stages from structure-of-arrays
+  // mirrors; nobody else reads them, so the cell build writes them only where it runs
   if (e.facc)
-    ok = ok && dalloc(e, &e.xs, e.mirrorN) == cudaSuccess &&
+    ok = ok && dalloc(e, &e.fqueue, 2) == cudaSuccess && dalloc(e, &e.xs, e.mirrorN) == cudaSuccess &&
          dalloc(e, &e.ys, e.mirrorN) == cudaSuccess &&
          dalloc(e, &e.zs, e.mirrorN) == cudaSuccess && dalloc(e, &e.ts, e.mirrorN) == cudaSuccess;
   if (!ok) {
@@ -817,7 +816,7 @@ int engine_setup_cells(Engine &e) {
   E_CUDA(cudaMemsetAsync(e.count, 0, sizeof(uint32_t) * C, e.stream));
   E_CUDA(cudaMemsetAsync(e.tcount, 0, sizeof(uint32_t) * e.ntile, e.stream));
   E_CUDA(cudaMemsetAsync(e.cctl, 0, sizeof(uint32_t) * 2, e.stream));
-  E_CUDA(cudaMemsetAsync(e.fqueue, 0, sizeof(uint32_t) * 2, e.stream));
+  if (e.fqueue) E_CUDA(cudaMemsetAsync(e.fqueue, 0, sizeof(uint32_t) * 2, e.stream));
   SysPlan *d_spl = nullptr;
   E_CUDA(engine_alloc_bytes(e, (void **)&d_spl, sizeof(SysPlan) * e.nsys));
   E_CUDA(cudaMemcpyAsync(d_spl, spl.data(), sizeof(SysPlan) * e.nsys, cudaMemcpyHostToDevice,

@@ -89,7 +89,7 @@ struct Engine {
   uint32_t nitems = 0;
   std::vector<uint32_t> item0, cell0;
   double *fpartials = nullptr;
-  uint32_t *fqueue = nullptr;  // the force kernel's item counter
+  uint32_t *fqueue = nullptr;  // the half-shell force kernel's item counter
   uint32_t cap_max = 0;
   uint32_t cap_half_max = 0;
   unsigned long long *facc = nullptr;  // half-shell force sums: fine and coarse, 2 x 3 x N

@@ -595,11 +595,9 @@ void make_block_map(const uint32_t *natoms, uint32_t nsys, BlockMap *map, uint32
   for (uint32_t s = 0; s < nsys; ++s) {
     blk0[s] = b;
     nblk[s] = blocks_for(natoms[s]);
-    const uint32_t per = kIntAtoms;
     for (uint32_t k = 0; k < nblk[s]; ++k) {
-      const uint32_t i0 = atom0 + k * per;
-      const uint32_t n = natoms[s] - k * per;
-      map[b++] = BlockMap{s, i0, n < per ? n : per, k};
+      const uint32_t first = k * kIntAtoms, n = natoms[s] - first;
+      map[b++] = BlockMap{s, atom0 + first, n < (uint32_t)kIntAtoms ? n : (uint32_t)kIntAtoms};
     }
     atom0 += natoms[s];
   }

@@ -45,9 +45,9 @@ struct SysInt {
 };
 
 // Block b of an integration launch covers atoms [i0, i0 + n) of system sys,
-// n <= kIntAtoms; it is block `k` of that system (i0 = first atom + k kIntAtoms).
+// n <= kIntAtoms; a system's blocks start at its first atom.
 struct BlockMap {
-  uint32_t sys, i0, n, k;
+  uint32_t sys, i0, n;
 };
 
 struct IntegrateArgs {
