@@ -100,3 +100,16 @@ def test_replica_rate_is_weak_scaling():
     spec.loader.exec_module(bench)
     one = bench.replica_rate(1, 1_048_576, 100, 0.0415)
     assert abs(bench.replica_rate(4, 1_048_576, 100, 0.0415) - 4 * one) < 1e-6 * one
+
+
+def test_reference_arm_without_the_reference_is_unavailable(po):
+    """Nothing else is timed in its place."""
+    if po.ref_available():
+        import pytest
+        pytest.skip("the reference's kernels are built here")
+    p = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference",
+                        "--gpus", "1", "--steps", "1", "--warmup", "3"],
+                       cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]
+    line = json.loads(p.stdout)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
