@@ -101,7 +101,7 @@ struct Stage {
   int z0, nz, nseg, periodic, overflow;
   int shifted;            // some frame shift is not zero
   int one;                // the system has one type, whatever the launch is compiled for
-  uint32_t nmax;          // largest norm of a home atom (float bits, non-negative)
+  uint32_t nmax;          // largest norm staged (float bits, non-negative)
   LJLocal<NT> lj;
   // several types: what the bound of a pair of types lies below the longest
   // one, per type of home atom as fp16 for candidate types 0 .. 3
@@ -490,7 +490,6 @@ template <int NT, int kWarps>
 __device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf, uint32_t *Ht, float *zb) {
   const uint32_t total = d.c0[9];
   const float cx = d.cx, cy = d.cy, cz = d.cz, sc = d.scale;
-  const uint32_t hb = d.hb, H = d.H;
   float nmax = 0.f;
   for (uint32_t u = threadIdx.x; u < total + 8u; u += kWarps * 32) {
     const float4 q = E[u];
@@ -509,7 +508,7 @@ __device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf,
     }
     const float far = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z));
     if (far < 1e29f && !isnan(n))
-      nmax = u - hb < H ? fmaxf(nmax, n) : nmax;
+      nmax = fmaxf(nmax, n);
     else
       E[u] = make_float4(kFar, kFar, kFar, q.w);
     const uint32_t k = u & 7u;
@@ -518,6 +517,17 @@ __device__ __forceinline__ void make_records(Stage<NT> &d, float4 *E, uint2 *Hf,
   }
   const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(nmax));
   if ((threadIdx.x & 31) == 0) atomicMax(&d.nmax, m);
+}
+
+// Whether a home atom of the item lies out of the range of the fp16 records (far outside
+// its cell); all threads of the CTA.  A norm out of that range is stored as infinity or
+// as what it is.
+template <int NT, int kWarps>
+__device__ __noinline__ bool home_out_of_range(const Stage<NT> &d, const float4 *E, const uint2 *Hf) {
+  bool out = false;
+  for (uint32_t u = d.hb + threadIdx.x; u < d.hb + d.H; u += kWarps * 32)
+    out = out || (unpack_half2(Hf[u].y).y > kMaxNorm && fabsf(E[u].x) < 1e29f);
+  return __syncthreads_or(out);
 }
 
 // One tile of 16 home atoms (one warp); energy sums (pe, shifted pe, virial,
@@ -880,7 +890,8 @@ __global__ void __launch_bounds__(kWarps * 32,
     __syncthreads();
   }
   // home atoms out of the range of fp16 records (far outside their cells): global path
-  const bool global = d.overflow || __uint_as_float(d.nmax) > kMaxNorm;
+  const bool global =
+      d.overflow || (__uint_as_float(d.nmax) > kMaxNorm && home_out_of_range<NT, kWarps>(d, E, Hf));
   const uint32_t ntile = d.ntile;
   double *ce = cle[ENERGY ? warp : 0];
   if (ENERGY && lane == 0)
