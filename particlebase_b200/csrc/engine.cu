@@ -128,8 +128,9 @@ namespace {
 // threads.  A frame read into a fresh allocation otherwise faults them one by one
 // inside the copy: 20 steps of the 2M-atom mixture and two 33 MB reads took
 // 30 ms, of which 8 ms were such faults; here they also pass while the GPU
-// still works.  Buffers whose pages are there cost one mincore call; smaller ones
-// (4 MB: 0.2 ms slower) do not pay for the threads.
+// still works.  Buffers whose pages are there cost a mincore call per 16 MB (one 2 MB
+// chunk in eight is looked at); smaller ones (4 MB: 0.2 ms slower) do not pay for the
+// threads.
 constexpr size_t kPopulateMin = 16u << 20, kPopulateChunk = 2u << 20;
 
 void populate_pages(void *host, size_t bytes) {

@@ -10,14 +10,15 @@
 // scratch: each atom's force is summed in registers and written once.
 //
 // Work items.  One CTA of 8 warps computes one work item = (system, x-y column
-// of cells, run of z cells [z0, z1)), about 8 tiles of 16 consecutive
-// (z-sorted) home atoms.  It stages the 3 x 3 neighbour columns over z cells
+// of cells, run of z cells [z0, z1)), at most about 8 tiles of 16 consecutive
+// (z-sorted) home atoms; at density 0.84 the shared memory makes it 7 cells of 14
+// atoms, 7 tiles.  It stages the 3 x 3 neighbour columns over z cells
 // [z0 - 1, z1] (periodic halo cells included) in shared memory by bulk copies
 // of the sorted positions (bounded wait), then a warp takes a tile and waits
 // for no other.  Four CTAs share an SM, so one's staging overlaps another's
 // computation.  What bounds it is instruction issue (70 % of the slots at 1M
-// atoms, shared memory 58 %).  Per home atom 182 warp instructions: staging 30,
-// block tables 23, phase 1 56, phase 2 73.  Longer runs stage fewer halo cells
+// atoms, shared memory 61 %).  Per home atom 188 warp instructions; when they were 186,
+// staging took 30, block tables and tile set-up 23, phase 1 56, phase 2 77.  Longer runs stage fewer halo cells
 // per home atom and shorter ones fit more CTAs: 4, 5, 6 and 7 cells of 14 atoms
 // took 0.362, 0.322, 0.284 and 0.268 ms at 1M atoms; 9 cells, at three CTAs per
 // SM, 0.293; CTAs of 16 warps over 14 cells 0.281.  A persistent kernel with
@@ -48,7 +49,7 @@
 // pairs inside the cutoff: about 4 % more.  With several types the indicators'
 // share of the product lowers the bound to that pair of types' own cutoff.
 // mma.sync and not tcgen05: a tile shares its window with no other, its product
-// has a depth of 8, and 52 of them take 8 % of the tensor pipe; the work is in
+// has a depth of 8, and 52 of them take 11 % of the tensor pipe; the work is in
 // reading their signs.  A lane owns 2 home atoms x 2 candidates of each block
 // and lists the candidates that may be near either of its two.
 //
@@ -65,7 +66,8 @@
 // the lanes, and windows and blocks depend on the item alone, so a system's
 // forces do not depend on scheduling or on the other systems of a batch.  An
 // item whose stage exceeds its capacity computes from global memory instead
-// (slower) and raises a status bit.
+// (slower) and raises a status bit; so does an item with a home atom out of the
+// range of the records (an open box, hundreds of sigma outside), without the bit.
 #include <cuda_fp16.h>
 
 #include <algorithm>

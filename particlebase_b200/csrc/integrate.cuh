@@ -16,7 +16,7 @@ constexpr int kIntThreads = 256;  // threads per integration block
 constexpr int kIntAtoms = 1024;   // atoms per integration block
 // A launch of few blocks (at most one per SM) takes one thread per atom instead of
 // 4 atoms per thread, with the same sums in the same order: a step of 32,000 atoms
-// 43.8 -> 39.5 us (Gaussian).  With more blocks the 256-thread form keeps
+// 43.8 -> 40.8 us (Gaussian).  With more blocks the 256-thread form keeps
 // more of them resident (1M atoms: 41 us against 58 with one atom per thread).
 constexpr uint32_t kIntWideBlocks = 148;
 

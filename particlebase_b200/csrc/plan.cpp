@@ -95,9 +95,8 @@ static int least_capacity(double atoms_per_cell, int seg) {
 }
 
 int choose_segment(double atoms_per_cell, int nz, double scale, int nt, bool half) {
-  // full-shell kernel: 8 tiles of 16 home atoms, one per warp of a CTA, with
-  // room for a few atoms above the mean; half-shell kernel: about 200 home
-  // atoms.  PB_FORCE_SEG overrides.  Shorter runs while the stage would not
+  // full-shell kernel: 124 home atoms, 8 tiles of 16 (one per warp of a CTA) with
+  // room for a few above the mean; half-shell kernel: about 200 home atoms.  PB_FORCE_SEG overrides.  Shorter runs while the stage would not
   // leave the CTAs per SM that the kernel's launch shape is built for.
   const double apc = std::max(atoms_per_cell, 1.0);
   int seg = half ? (int)std::lround(200.0 * scale / apc) : (int)std::lround(124.0 * scale / apc);

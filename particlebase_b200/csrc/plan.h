@@ -26,9 +26,10 @@ void morton_columns(int nx, int ny, std::vector<uint32_t> &rank, std::vector<uin
 // neighbour outside the grid is kNoCell.
 void neighbor_table(const Grid &g, std::vector<uint32_t> &out);
 
-// z cells per force work item for a mean cell occupancy: about 119 * scale
+// z cells per force work item for a mean cell occupancy: about 124 * scale
 // home atoms per item (8 tiles of 16), at most force_max_segment(), and short
-// enough for four force CTAs per SM with `nt` atom types.
+// enough for the CTAs per SM of the launch shape (four with one atom type, three
+// with more): at 14 atoms a cell and one type 7 cells, 98 atoms.
 // `half`: the half-shell force kernel runs (about 200 * scale home atoms; its
 // stage has to fit as well).
 int choose_segment(double atoms_per_cell, int nz, double scale = 1.0, int nt = 1,

@@ -3,7 +3,7 @@
 The force kernel's work item is one column run of `seg` z cells of one
 system (its cell tile: 3 x 3 columns x (seg + 2) cells staged in shared
 memory); `seg` is chosen per system from its mean cell occupancy to give
-about 160 home atoms per CTA, times a scale.  The tuner times whole steps of
+about 124 home atoms per CTA, times a scale.  The tuner times whole steps of
 the batch for each (threads, scale) candidate and keeps the fastest.  Both
 parameters change only how the work is split into CTAs, not which pairs are
 computed.  Results are cached in a JSON file keyed by the device name, the

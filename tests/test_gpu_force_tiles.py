@@ -2,7 +2,8 @@
 all pairs in FP64: partial and single-atom tiles, empty cells, columns of one
 and of many runs, cells wider than the cutoff (more candidate blocks than the
 warps' table holds), one to five atom types with their own cutoffs, 64-bit
-sums, open boxes, and atoms far outside their cells."""
+sums, open boxes, atoms far outside their cells on every side, pairs that do
+not interact, the soft core, and uneven density."""
 import numpy as np
 import pytest
 
@@ -90,7 +91,7 @@ def test_cells_wider_than_the_cutoff(cuda_lib, rmax, ntypes):
 @pytest.mark.parametrize("far", [0.0, 30.0, 4000.0])
 def test_open_box_and_atoms_far_outside(cuda_lib, far):
     """Past some hundred cell edges an atom leaves the range of the stage's fp16
-    records, and the items that stage it compute from global memory."""
+    records, and the items whose home atom it is compute from global memory."""
     s = system((12.0, 11.0, 14.0), 700, 1, 5)
     if far:
         s.r[3] = (-far, 4.0, 5.0)

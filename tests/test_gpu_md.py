@@ -375,8 +375,7 @@ def test_open_box_rejects_half_shell_and_lists(cuda_lib, golden):
 
 def test_empty_cells_and_crowded_cells(cuda_lib, po):
     """Sparse gas with many empty cells plus a clump of 60 atoms in one cell:
-    exercises empty ranges, the >32-member cell ordering and the global-memory
-    fallback of the force kernel when its shared-memory stage overflows."""
+    exercises empty ranges and the >32-member cell ordering."""
     rng = np.random.default_rng(2)
     L = 30.0
     gas = rng.uniform(0, L, (800, 3))
@@ -480,8 +479,8 @@ def test_runs_of_odd_length_match_one_run(cuda_lib, gaussian):
 
 def test_wait_timeout_is_reported_and_the_handle_recovers(cuda_lib, po):
     """Failure detection without a GPU fault: a test hook makes the force
-    kernel's producer warps withhold their first hand-off, so the consumer
-    warps' bounded wait (2,000 polls of at most 1 us) runs out.  The call
+    kernel withhold the copies of its stage, so the bounded wait for them
+    (2,000 polls of at most 1 us) runs out.  The call
     returns, PB_STATUS_WAIT_TIMEOUT is set, and the next force call on the
     same handle is complete and correct."""
     s = perturbed(W.config_c1(), 0.05, 3)
