@@ -72,7 +72,8 @@ typedef enum pb_field {
   PB_FIELD_F = 3,          /* float4[N]   force F(t)                      (get/set) */
   PB_FIELD_FOLD = 4,       /* float4[N]   previous force (VV Fold)        (get/set) */
   PB_FIELD_MINV = 5,       /* float[N]    1/mass                          (get/set) */
-  PB_FIELD_TYPE = 6,       /* uint16[N]   type id                         (get/set) */
+  PB_FIELD_TYPE = 6,       /* uint16[N]   type id; 8 and more are labels that only
+                              one-type systems take (get/set) */
   PB_FIELD_CELL_OF = 7,    /* uint32[N]   reference cell id of each atom  (get) */
   PB_FIELD_PID = 8,        /* uint32[N]   particle id per sorted slot     (get) */
   PB_FIELD_CELL_START = 9, /* uint32[C+1] first slot of each cell, in key order (get) */
